@@ -684,9 +684,21 @@ constexpr int BASIS_NODES = 40;
 constexpr int MMA_SYN_TILES = 9;   // 3 node tiles (48 rows) x 3 coefficient tiles (24 columns)
 constexpr int MMA_PB_TILES = 10;   // 2 coefficient tiles (32 rows) x 5 node tiles (40 columns)
 constexpr int MMA_TABLE_FLOATS = (MMA_SYN_TILES + MMA_PB_TILES) * 2 * 32 * 4;
+// FP64 (fcc_forces64.cuh): columns of the contraction matrix, its rows after
+// the last node, neighbour records staged per body and doubles between staged
+// records (208 bytes: the 16-byte reads of a warp's lanes at different
+// neighbours fall into different banks).  With NBMAX64 = 10 two blocks of 224
+// threads fit an SM's shared memory (14 warps); 12 would not.
+constexpr int M64_COLS = 20, M64_PAD = 80, NBMAX64 = 8, SREC64 = RECW + 2;
+// own body-frame coefficients, sin and cos of theta, 1/(2 a0)
+constexpr int SCF64 = NCM + 3;
+// nodes whose rows of the FP64 matrix a block holds: one chunk, or up to two
+// (more are read where they are)
+__host__ __device__ constexpr int m64_rows(bool one) { return one ? BASIS_NODES : 2 * BASIS_NODES; }
 template <class T>
-__host__ __device__ constexpr size_t basis_table_bytes() {
-    return sizeof(T) == 4 ? (size_t)BASIS_NODES * KM * 4 * sizeof(T) + (size_t)MMA_TABLE_FLOATS * sizeof(float) : 0;
+__host__ __device__ constexpr size_t basis_table_bytes(bool one) {
+    return sizeof(T) == 4 ? ((size_t)BASIS_NODES * (KM * 4 + 2) + (size_t)MMA_TABLE_FLOATS) * sizeof(float)
+                          : (size_t)m64_rows(one) * (M64_COLS + 2) * sizeof(T);
 }
 
 // Per warp: the own records of its 32/L bodies, then NBMAX neighbour
@@ -708,7 +720,16 @@ __host__ __device__ constexpr size_t walk_bytes_per_warp() {
 }
 template <class T, int L>
 __host__ __device__ constexpr size_t stage_bytes_per_warp() {
+    // FP64: 4 own and 4 x NBMAX64 neighbour records, the nodes' offsets and pressures, the own coefficients
+    if (sizeof(T) == 8) return (4 * (1 + NBMAX64) * SREC64 + 3 * 5 * 32 + 4 * SCF64) * sizeof(T);
     return (size_t)(32 / L) * (1 + NBMAX) * RECW * sizeof(T) + desc_slot_bytes<T>() + walk_bytes_per_warp<T, L>();
+}
+
+// the walk slots' place in a warp's stage (draw_ahead)
+template <class T, int L>
+__host__ __device__ constexpr int draw_ahead_slot() {
+    return sizeof(T) == 8 ? 4 * (1 + NBMAX64) * SREC64
+                          : (32 / L) * (1 + NBMAX) * RECW + (int)(desc_slot_bytes<T>() / sizeof(T));
 }
 
 // ------------------------------------------------ tensor-core contractions
@@ -941,6 +962,29 @@ __device__ __forceinline__ void cis_pow(T c1, T s1, int n, T& cn, T& sn) {
     cn = rc;
     sn = rs;
 }
+// FP64: the same with the products that are fused written out, so that every
+// kernel rounds alike, and without branches
+__device__ __forceinline__ double mode_norm(double a, double b) { return sqrt_normal(fma(a, a, b * b)); }
+__device__ __forceinline__ double mode_sq(double a, double b) { return fma(a, a, b * b); }
+__device__ __forceinline__ void to_lab(double a, double b, double co, double so, double& al, double& be) {
+    al = fma(a, co, -(b * so));
+    be = fma(a, so, b * co);
+}
+__device__ __forceinline__ void cis_pow(double c1, double s1, int n, double& cn, double& sn) {
+    double rc = 1.0, rs = 0.0, bc = c1, bs = s1;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const double pc = fma(rc, bc, -(rs * bs)), ps = fma(rc, bs, rs * bc);
+        const bool on = n & (1 << b);
+        rc = on ? pc : rc;
+        rs = on ? ps : rs;
+        const double t = fma(bc, bc, -(bs * bs));
+        bs = 2.0 * bc * bs;
+        bc = t;
+    }
+    cn = rc;
+    sn = rs;
+}
 
 // Translational displacement of a body with substrate drag, plus the forces
 // of its children with parent drag (src/dynamics.jl:84-99).
@@ -1019,44 +1063,63 @@ __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T
     const T dtmu = dt * P.muab[ti];
     const int K = P.K;
     const int Kt = min(K, P.kmax[ti]);  // modes of this type; the rest stay zero
-    T an[MPL], bn[MPL];
-    double sp = 0.0;
+    // Every lane computes its MPL modes without branches (those of a lane
+    // beyond Kt give zero), so their chains overlap; a simulation whose modes
+    // fit one per lane skips the second
+    T an[MPL], bn[MPL], nrm[MPL];
+    double sp = 0.0, qp = 0.0;
+    T bp = T(0);
 #pragma unroll
     for (int u = 0; u < MPL; ++u) {
+        an[u] = bn[u] = nrm[u] = T(0);
+        if (u > 0 && K <= u * L) continue;  // uniform
         const int m = l + u * L;
-        an[u] = T(0);
-        bn[u] = T(0);
-        if (m < Kt) {
-            const T ga = gA[u] * r0, gb = gB[u] * r0;
-            T so, co;
-            cis_pow(co1, so1, m + 2, co, so);
-            const T a = pre.a[u], b = pre.b[u];
-            const T gca = ga * co + gb * so - h0 * a;
-            const T gcb = -ga * so + gb * co - h0 * b;
-            an[u] = a - dtmu * gca;
-            bn[u] = b - dtmu * gcb;
-            sp += (double)mode_norm(an[u], bn[u]);
-        }
+        const bool on = m < Kt;
+        const T ga = gA[u] * r0, gb = gB[u] * r0;
+        T so, co;
+        cis_pow(co1, so1, m + 2, co, so);
+        const T a = pre.a[u], b = pre.b[u];
+        const T gca = ga * co + gb * so - h0 * a;
+        const T gcb = -ga * so + gb * co - h0 * b;
+        const T a1 = a - dtmu * gca, b1 = b - dtmu * gcb;
+        an[u] = on ? a1 : T(0);
+        bn[u] = on ? b1 : T(0);
+        nrm[u] = mode_norm(an[u], bn[u]);
     }
-    // enforce_shape! (src/dynamics.jl:44-64) with FP64 sums
-    const double ssum = group_sum<L>(sp);
-    if (ssum > SHAPE_BOUND) {
-        const double f = SHAPE_BOUND / ssum;
+    // enforce_shape! (src/dynamics.jl:44-64) with FP64 sums: the three sums of
+    // the shape as it is at once; a body beyond the bound (rare) is scaled and
+    // summed again
+    auto sums = [&] {
+        sp = qp = 0.0;
+        bp = T(0);
 #pragma unroll
         for (int u = 0; u < MPL; ++u) {
-            an[u] = T((double)an[u] * f);
-            bn[u] = T((double)bn[u] * f);
+            if (u > 0 && K <= u * L) continue;
+            sp += (double)nrm[u];
+            qp += mode_sq(an[u], bn[u]);
+            bp += nrm[u];
         }
-    }
-    double qp = 0.0;
+        sp = group_sum<L>(sp);
+        qp = group_sum<L>(qp);
+        bp = group_sum<L>(bp);
+    };
+    sums();
+    if (__any_sync(FULL, sp > SHAPE_BOUND)) {
+        if (sp > SHAPE_BOUND) {
+            const double f = SHAPE_BOUND / sp;
 #pragma unroll
-    for (int u = 0; u < MPL; ++u) qp += mode_sq(an[u], bn[u]);
-    const double qs = group_sum<L>(qp);
-    const T a0n = T(sqrt(1.0 - qs * 0.5));
+            for (int u = 0; u < MPL; ++u) {
+                an[u] = T((double)an[u] * f);
+                bn[u] = T((double)bn[u] * f);
+                nrm[u] = mode_norm(an[u], bn[u]);
+            }
+        }
+        sums();
+    }
+    const T a0n = T(sqrt(1.0 - qp * 0.5));
 
     // lab frame of the new state (src/geometry.jl:208-227)
     T* rn = rec_next(d, par) + (size_t)(act ? g : 0) * RECW;
-    T bp = T(0);
 #pragma unroll
     for (int u = 0; u < MPL; ++u) {
         const int m = l + u * L;
@@ -1064,7 +1127,6 @@ __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T
             T so, co, al, be;
             cis_pow(cn1, sn1, m + 2, co, so);
             to_lab(an[u], bn[u], co, so, al, be);
-            bp += mode_norm(an[u], bn[u]);
             if (act) {
                 rn[r_al(m)] = r0 * al;
                 rn[r_be(m)] = r0 * be;
@@ -1073,7 +1135,7 @@ __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T
             }
         }
     }
-    const T rmax = r0 * (a0n + group_sum<L>(bp));
+    const T rmax = r0 * (a0n + bp);
 
     if (act && l == 0) {
         T dxp, dyp;
@@ -1141,6 +1203,173 @@ __device__ __forceinline__ void carry_record_staged(const DevPtrs<T>& d, int g, 
 // ==================================================== force evaluation ==
 enum : int { MODE_FUSED = 0, MODE_FORCES = 1, MODE_DIAG = 2 };
 
+// Body terms of the contour integral Q: W = sum_t dF_t/dQ * dphi, the energy
+// E = e_1 + (e_2 + ...) (src/energies/body_terms.jl:8-34).
+template <class T>
+__device__ __forceinline__ void body_terms(const SimDesc<T>& P, int ti, T Q, T r0, T dphi, T& W, T& E) {
+    W = E = T(0);
+    const int nbt = P.nbt;
+    // the first NB terms without branches, their parameters read at once (a
+    // loop over them waited for shared memory at every term and cost 700
+    // cycles of a warp group's 14 700 at two terms)
+    constexpr int NB = 4;
+    T a[NB], b[NB];
+    bool on[NB], ten[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        a[q] = P.bt_a[q];
+        b[q] = P.bt_b[q];
+        on[q] = q < nbt && (P.bt_mask[q] & (1u << ti));
+        ten[q] = P.bt_kind[q] == BT_TENSION;
+    }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        const T v = ten[q] ? a[q] : a[q] * (T(2) * (Q - b[q] * r0));
+        W = on[q] ? W + v : W;
+    }
+    for (int q = NB; q < nbt; ++q) {
+        if (!(P.bt_mask[q] & (1u << ti))) continue;
+        const T aq = P.bt_a[q];
+        W += P.bt_kind[q] == BT_TENSION ? aq : aq * (T(2) * (Q - P.bt_b[q] * r0));
+    }
+    for (int q = nbt - 1; q >= NB; --q) {
+        if (!(P.bt_mask[q] & (1u << ti))) continue;
+        const T aq = P.bt_a[q];
+        const T dq = Q - P.bt_b[q] * r0;
+        E = (P.bt_kind[q] == BT_TENSION ? aq * Q : aq * (dq * dq)) + E;
+    }
+#pragma unroll
+    for (int q = NB - 1; q >= 0; --q) {
+        const T dq = Q - b[q] * r0;
+        const T v = ten[q] ? a[q] * Q : a[q] * (dq * dq);
+        E = on[q] ? v + E : E;
+    }
+    W *= dphi;
+}
+
+// User body terms of one body (include/fcc_user_terms.h), one contour chunk:
+// the integrals Q_j of their integrands over the nodes, then the node weights
+// w = dF/dQ_j dphi and the energies F(Q).
+template <class T>
+struct UserBody {
+    T Q[MUT][fcc_user::MAX_M], w[MUT][fcc_user::MAX_M];
+    static __device__ __forceinline__ bool on(const SimDesc<T>& P, int u, int ti) {
+        return u < P.nub && ((P.ub_mask[u] >> ti) & 1u);
+    }
+    template <int L, int S>
+    __device__ __forceinline__ void integrals(const SimDesc<T>& P, int ti, unsigned vmask, const T (&R)[S],
+                                              const T (&R1)[S], const T (&R2)[S], T dphi) {
+#pragma unroll
+        for (int u = 0; u < MUT; ++u) {
+#pragma unroll
+            for (int j = 0; j < fcc_user::MAX_M; ++j) Q[u][j] = T(0);
+            if (!on(P, u, ti)) continue;
+#pragma unroll
+            for (int sl = 0; sl < S; ++sl)
+                if (vmask & (1u << sl)) {
+                    T q[fcc_user::MAX_M] = {};
+                    fcc_user::body_q<T>(P.ub_id[u], R[sl], R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], q);
+#pragma unroll
+                    for (int j = 0; j < fcc_user::MAX_M; ++j) Q[u][j] += q[j];
+                }
+        }
+        // every lane of the warp takes the shuffles (a warp may hold bodies of several types)
+#pragma unroll
+        for (int u = 0; u < MUT; ++u)
+            if (u < P.nub) {
+#pragma unroll
+                for (int j = 0; j < fcc_user::MAX_M; ++j) Q[u][j] = group_sum<L>(Q[u][j]) * dphi;
+            }
+    }
+    __device__ __forceinline__ void energies(const SimDesc<T>& P, int ti, T r0, T dphi, T& E) {
+#pragma unroll
+        for (int u = 0; u < MUT; ++u) {
+#pragma unroll
+            for (int j = 0; j < fcc_user::MAX_M; ++j) w[u][j] = T(0);
+            if (!on(P, u, ti)) continue;
+            T dF[fcc_user::MAX_M] = {};
+            fcc_user::body_dF<T>(P.ub_id[u], Q[u], r0, ti + 1, P.ub_a[u], P.ub_b[u], dF);
+#pragma unroll
+            for (int j = 0; j < fcc_user::MAX_M; ++j) w[u][j] = dF[j] * dphi;
+            E += fcc_user::body_F<T>(P.ub_id[u], Q[u], r0, ti + 1, P.ub_a[u], P.ub_b[u]);
+        }
+    }
+    __device__ __forceinline__ void gradients(const SimDesc<T>& P, int ti, T r, T r1, T r2, T& GR, T& GD, T& GDD) const {
+#pragma unroll
+        for (int u = 0; u < MUT; ++u) {
+            if (!on(P, u, ti)) continue;
+            T dq[fcc_user::MAX_M][3] = {};
+            fcc_user::body_dq<T>(P.ub_id[u], r, r1, r2, P.ub_a[u], P.ub_b[u], dq);
+#pragma unroll
+            for (int j = 0; j < fcc_user::MAX_M; ++j) {
+                GR += w[u][j] * dq[j][0];
+                GD += w[u][j] * dq[j][1];
+                GDD += w[u][j] * dq[j][2];
+            }
+        }
+    }
+};
+
+// Pressure of the user contact terms at depth dd against a body with record
+// word wj.
+template <class T>
+__device__ __forceinline__ T user_pressure(const SimDesc<T>& P, T dd, int ti, int wj, int pi) {
+    T gv = T(0);
+#pragma unroll
+    for (int u = 0; u < MUT; ++u)
+        if (u < P.nuc && ((P.uc_mask[u] >> ti) & 1u))
+            gv += fcc_user::contact_g<T>(P.uc_id[u], dd, ti + 1, (wj & 7) + 1, (wj >> 3) == pi, P.uc_a[u], P.uc_b[u]);
+    return gv;
+}
+
+// Bond forces on the centre of body g (src/energies/bonds.jl:98-111), by
+// every lane of the body, no shuffles.
+template <class T, bool USER>
+__device__ __forceinline__ void bond_forces(const DevPtrs<T>& d, const SimDesc<T>& P, const T* rc, int g, int ti, T xi,
+                                            T yi, T& fx, T& fy) {
+    if (!(P.nbd > 0 || (USER && P.nubd > 0))) return;
+    const int bc = __ldg(d.bd_count + g);
+    T bx = T(0), by = T(0);
+    for (int q = 0; q < bc; ++q) {
+        const int j = __ldg(d.bd_idx + (size_t)g * d.bcap + q);
+        T xj, yj, rmj, wj;
+        load_head(rc + (size_t)j * RECW, xj, yj, rmj, wj);
+        const int tj = unpack_w(wj) & 7;
+        const T d0 = minimum_image_exact(sub_rn(xi, xj), P.Lx);
+        const T d1 = minimum_image_exact(sub_rn(yi, yj), P.Ly);
+        T a0 = T(0), a1 = T(0);
+        for (int u = P.nbd - 1; u >= 0; --u) {
+            const uint32_t mk = P.bd_mask[u];
+            if (!((mk >> ti) & 1u) || !((mk >> tj) & 1u)) continue;
+            const T rr = t_sqrt(d0 * d0 + d1 * d1);
+            const T k = P.bd_k[u], rb = P.bd_r0[u];
+            const T f = rr > T(0) ? k * (T(1) - rb / rr) : (rb == T(0) ? k : T(0));
+            a0 = f * d0 + a0;
+            a1 = f * d1 + a1;
+        }
+        if constexpr (USER) {
+#pragma unroll
+            for (int u = 0; u < MUT; ++u) {
+                if (u >= P.nubd || !((P.ubd_mask[u] >> ti) & 1u) || !((P.ubd_mask[u] >> tj) & 1u)) continue;
+                T hx, hy;
+                fcc_user::bond_grad<T>(P.ubd_id[u], d0, d1, ti + 1, tj + 1, P.ubd_a[u], P.ubd_b[u], hx, hy);
+                a0 += hx;
+                a1 += hy;
+            }
+        }
+        bx += a0;
+        by += a1;
+    }
+    fx += bx;
+    fy += by;
+}
+
+}  // namespace fcc
+
+#include "fcc_forces64.cuh"
+
+namespace fcc {
+
 // Forces on the 32/L bodies of warp group `wg`, and in MODE_FUSED their
 // update.  `stage` is this warp's shared-memory slot for neighbour records.
 // Follows, per body i:
@@ -1155,7 +1384,7 @@ enum : int { MODE_FUSED = 0, MODE_FORCES = 1, MODE_DIAG = 2 };
 // pressures and bond gradients are added, and the pullback includes R''.
 template <class T, int L, int S, bool ONE, int MODE, bool USER = false>
 __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stage, int par, const SimDesc<T>* sim0,
-                                            const T* tab, int& cached, int* rbp, const BarrierLocal* lone) {
+                                            const T* tab, int& cached, int* rbp, const BarrierLocal* lone, bool drawn) {
     constexpr int BPW = 32 / L;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int CH16 = RECW * (int)sizeof(T) / 16;  // 16-byte chunks per record
@@ -1226,8 +1455,12 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     // ---- Philox normals of this body and step, early so their latency hides
     // behind the loads: lane 1 draws block 0 (translation), the other lanes
     // block 1 (orientation) (src/random.jl:75-100)
+    // (or during the last step barrier: draw_ahead)
     T nz[2] = {T(0), T(0)};
-    if (MODE == MODE_FUSED && P.has_noise)
+    if (MODE == MODE_FUSED && drawn) {
+        const T* ahead = stage + draw_ahead_slot<T, L>() + lane;
+        nz[0] = ahead[0], nz[1] = ahead[32];
+    } else if (MODE == MODE_FUSED && P.has_noise)
         philox_pair<T>(P.k0, P.k1, (uint32_t)(gg - P.body_off + 1), (uint64_t)clk, l == 1 ? 0u : 1u, nz[0], nz[1]);
 
     // ---- stage the neighbour records in shared memory (cp.async)
@@ -1289,8 +1522,15 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         for (int sl = 0; sl < S; ++sl) {
             const int k = ch * L * S + l + L * sl;
             const bool v = k < nth;
-            const T c1 = v ? __ldg(d.cs + 2 * k) : T(1);
-            const T s1 = v ? __ldg(d.cs + 2 * k + 1) : T(0);
+            T c1 = T(1), s1 = T(0);
+            if constexpr (USE_TAB) {
+                const float2 e = reinterpret_cast<const float2*>(tab + BASIS_NODES * KM * 4 + MMA_TABLE_FLOATS)[v ? k : 0];
+                c1 = v ? e.x : T(1);
+                s1 = v ? e.y : T(0);
+            } else if (v) {
+                c1 = __ldg(d.cs + 2 * k);
+                s1 = __ldg(d.cs + 2 * k + 1);
+            }
             C1[sl] = c1;
             S1[sl] = s1;
             cc[sl] = c1;
@@ -1364,22 +1604,8 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     }
 
     // ---- body terms: W = sum_t dF_t/dQ * dphi, E = e_1 + (e_2 + ...)
-    T W = T(0), E = T(0);
-    {
-        const int nbt = P.nbt;
-        for (int q = 0; q < nbt; ++q) {
-            if (!(P.bt_mask[q] & (1u << ti))) continue;
-            const T a = P.bt_a[q];
-            W += P.bt_kind[q] == BT_TENSION ? a : a * (T(2) * (Q - P.bt_b[q] * r0));
-        }
-        for (int q = nbt - 1; q >= 0; --q) {
-            if (!(P.bt_mask[q] & (1u << ti))) continue;
-            const T a = P.bt_a[q];
-            const T dq = Q - P.bt_b[q] * r0;
-            E = (P.bt_kind[q] == BT_TENSION ? a * Q : a * (dq * dq)) + E;
-        }
-        W *= dphi;
-    }
+    T W, E;
+    body_terms(P, ti, Q, r0, dphi, W, E);
     // user body terms: energies F_u(Q) and node weights UW = dF_u/dQ_j dphi
     T UW[MUT][fcc_user::MAX_M];
     if constexpr (USER) {
@@ -1737,6 +1963,30 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
                       rbp);
 }
 
+// The force evaluation of a precision.
+template <class T, int L, int S, bool ONE, int MODE, bool USER>
+__device__ __forceinline__ void forces_group(const DevPtrs<T>& d, int wg, T* stage, int par, const SimDesc<T>* sim0,
+                                             const T* tab, int& cached, int* rbp, const BarrierLocal* lone,
+                                             bool drawn) {
+    if constexpr (sizeof(T) == 8) forces_warp64<ONE, MODE, USER>(d, wg, stage, par, sim0, tab, rbp, lone, drawn);
+    else forces_warp<T, L, S, ONE, MODE, USER>(d, wg, stage, par, sim0, tab, cached, rbp, lone, drawn);
+}
+
+// Normals of warp group wg's bodies in draw clk of a lone simulation, left in
+// the warp's walk slots (free between steps) for the forces of the next step:
+// drawn while the block waits at the step barrier, they cost no step time.
+template <class T, int L>
+__device__ __forceinline__ void draw_ahead(const DevPtrs<T>& d, int wg, T* stage, const SimDesc<T>& P, long long clk) {
+    const int lane = threadIdx.x & 31, l = lane & (L - 1);
+    const int g = wg * (32 / L) + lane / L;
+    const int gg = g < d.Ntot ? g : 0;
+    T z0, z1;
+    philox_pair<T>(P.k0, P.k1, (uint32_t)(gg - P.body_off + 1), (uint64_t)clk, l == 1 ? 0u : 1u, z0, z1);
+    T* ahead = stage + draw_ahead_slot<T, L>() + lane;
+    ahead[0] = z0;
+    ahead[32] = z1;
+}
+
 // Phase B of the split step: displacement with parent drag + update of the
 // bodies of warp group `wg`, from the forces phase A stored.
 template <class T, int L>
@@ -1924,32 +2174,45 @@ __device__ __forceinline__ const SimDesc<T>* copy_desc(const DevPtrs<T>& d) {
 
 // Dynamic shared memory of the force kernels: the FP32 mode table (one
 // contour chunk of nodes), then one neighbour stage per warp.
-template <class T>
+template <class T, bool ONE>
 __device__ __forceinline__ T* warp_stage(size_t bytes_per_warp) {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
-    return reinterpret_cast<T*>(fcc_smem + basis_table_bytes<T>() + (threadIdx.x >> 5) * bytes_per_warp);
+    return reinterpret_cast<T*>(fcc_smem + basis_table_bytes<T>(ONE) + (threadIdx.x >> 5) * bytes_per_warp);
 }
 // the whole stage area of the block (every warp's stage, in order)
-template <class T>
+template <class T, bool ONE>
 __device__ __forceinline__ unsigned char* block_stage_of() {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
-    return fcc_smem + basis_table_bytes<T>();
+    return fcc_smem + basis_table_bytes<T>(ONE);
 }
 
-// Copy the mode table of the first min(nth, BASIS_NODES) nodes, and after it
-// the tensor-core fragment table, into shared memory (FP32 single-chunk
-// kernels); returns the mode table, or null when unused.
+// Copy the tables of a single-chunk kernel into shared memory: FP32 the mode
+// table of the first min(nth, BASIS_NODES) nodes and after it the tensor-core
+// fragment table, FP64 the contraction matrix and the nodes' (cos, sin).
+// Returns the table, or null when unused.
 template <class T, bool ONE>
 __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
-    if (!(sizeof(T) == 4 && ONE)) return nullptr;
     T* tab = reinterpret_cast<T*>(fcc_smem);
+    if constexpr (sizeof(T) == 8) {  // M, then the nodes' (cos, sin)
+        constexpr int rows = m64_rows(ONE);
+        if (d.nth > rows) return nullptr;
+        for (int u = threadIdx.x; u < rows * M64_COLS; u += blockDim.x) tab[u] = __ldg(d.basis + u);
+        for (int u = threadIdx.x; u < 2 * d.nth; u += blockDim.x) tab[rows * M64_COLS + u] = __ldg(d.cs + u);
+        __syncthreads();
+        return tab;
+    }
+    if (!ONE) return nullptr;
     const int n = min(d.nth, BASIS_NODES) * KM * 4;
     for (int u = threadIdx.x; u < n; u += blockDim.x) tab[u] = __ldg(d.basis + u);
     if (d.mtab) {  // the tensor-core fragments follow the mode table
         float* mt = reinterpret_cast<float*>(fcc_smem) + BASIS_NODES * KM * 4;
         for (int u = threadIdx.x; u < MMA_TABLE_FLOATS; u += blockDim.x) mt[u] = __ldg(d.mtab + u);
     }
+    // and the nodes' (cos, sin): an acquire at a grid barrier empties L1, so
+    // read from global memory they cost a trip to L2 every step
+    for (int u = threadIdx.x; u < 2 * min(d.nth, BASIS_NODES); u += blockDim.x)
+        tab[BASIS_NODES * KM * 4 + MMA_TABLE_FLOATS + u] = __ldg(d.cs + u);
     __syncthreads();
     return tab;
 }
@@ -1960,14 +2223,14 @@ __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
 // each warp its first and then the block's next untaken one.
 template <class T, int L, int S, bool ONE, bool SPLIT, int BLK, int MINB, bool USER = false>
 __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, int par0) {
-    constexpr int WPB = BLK / 32;
+    const int WPB = blockDim.x >> 5;  // at most BLK / 32
     const int warp = threadIdx.x >> 5;
     const int ngroups = (d.Ntot + (32 / L) - 1) / (32 / L);
     const int g0 = (int)((long long)ngroups * blockIdx.x / gridDim.x);
     const int g1 = (int)((long long)ngroups * (blockIdx.x + 1) / gridDim.x);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
-    T* stage = warp_stage<T>(stage_bytes_per_warp<T, L>());
+    T* stage = warp_stage<T, ONE>(stage_bytes_per_warp<T, L>());
     const T* tab = stage_basis<T, ONE>(d);
     const SimDesc<T>* sim0 = copy_desc(d);
     __shared__ BarrierLocal bl;
@@ -1983,12 +2246,16 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
     __shared__ int s_next[2];  // next untaken warp group of the block, per step parity
     if (dyn && threadIdx.x == 0) s_next[0] = g0 + WPB;
     __syncthreads();
+    // a lone simulation's warps draw the normals of their first group of the
+    // next step while they wait at the step barrier
+    const bool ahead = FCC_FLAT_BARRIER && !SPLIT && !USER && lone && sim0->has_noise;
+    bool drawn = false;
     for (int st = 0; st < nsteps; ++st) {
         const int par = (par0 + st) & 1;
         if (bl.any) {
             // the work list of a pool lives in the warps' stage area, free
             // between the closing barrier of a step and the forces
-            if (!rebuild_prologue(d, par, tid, nthr, bl, sim0, reinterpret_cast<int*>(block_stage_of<T>()),
+            if (!rebuild_prologue(d, par, tid, nthr, bl, sim0, reinterpret_cast<int*>(block_stage_of<T, ONE>()),
                                   (int)(WPB * stage_bytes_per_warp<T, L>() / sizeof(int))))
                 return;
             cached = -1;  // the descriptor slots were overwritten
@@ -1998,24 +2265,27 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
             // next untaken group (groups cost unequal time: contacts, hits)
             if (threadIdx.x == 0) s_next[(st + 1) & 1] = g0 + WPB;  // last used by the previous step
             for (int wg = g0 + warp; wg < g1;) {
-                forces_warp<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER>(d, wg, stage, par, sim0, tab,
+                forces_group<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER>(d, wg, stage, par, sim0, tab,
                                                                                    cached, &bl.rebuild,
-                                                                                   lone ? &bl : nullptr);
+                                                                                   lone ? &bl : nullptr,
+                                                                                   drawn && wg == g0 + warp);
                 int nx = 0;
                 if ((threadIdx.x & 31) == 0) nx = atomicAdd(&s_next[st & 1], 1);
                 wg = __shfl_sync(0xffffffffu, nx, 0);
             }
         } else {
             for (int wg = g0 + warp; wg < g1; wg += WPB)
-                forces_warp<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER>(d, wg, stage, par, sim0, tab,
+                forces_group<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER>(d, wg, stage, par, sim0, tab,
                                                                                    cached, &bl.rebuild,
-                                                                                   lone ? &bl : nullptr);
+                                                                                   lone ? &bl : nullptr,
+                                                                                   drawn && wg == g0 + warp);
         }
         if (SPLIT) {
             if (!grid_barrier(d.sync, bl, [](unsigned) { return -1; })) return;
             for (int wg = g0 + warp; wg < g1; wg += WPB) update_warp_split<T, L>(d, wg, par, sim0, &bl.rebuild);
         }
         const int f0 = bl.flags;  // fixed during the step (read before thread 0 may rewrite it)
+        const long long c0 = bl.clock;
         __syncthreads();          // every warp's skin verdict is in bl.rebuild
         unsigned rb = 0;
         if (threadIdx.x == 0) {  // reported with the arrival; cleared before the next forces phase
@@ -2039,7 +2309,11 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
                 bl.flags = (code >> 1) & 0xff;
                 bl.clock += tick;
             };
-            if (!flat_barrier(d.sync, bl, rb, decide, false)) return;
+            auto shadow = [&] {
+                if (ahead && g0 + warp < g1 && st + 1 < nsteps) draw_ahead<T, L>(d, g0 + warp, stage, *sim0, c0 + tick);
+            };
+            if (!flat_barrier(d.sync, bl, rb, decide, false, shadow)) return;
+            drawn = ahead;
             continue;
         }
         if (!grid_barrier(
@@ -2074,11 +2348,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_gradients(DevPt
     const int wpb = blockDim.x >> 5;
     const int wg = blockIdx.x * wpb + (threadIdx.x >> 5);
     const int ngroups = (d.Ntot + (32 / L) - 1) / (32 / L);
-    T* stage = warp_stage<T>(stage_bytes_per_warp<T, L>());
+    T* stage = warp_stage<T, ONE>(stage_bytes_per_warp<T, L>());
     const T* tab = stage_basis<T, ONE>(d);
     const SimDesc<T>* sim0 = copy_desc(d);
     int cached = -1;
-    if (wg < ngroups) forces_warp<T, L, S, ONE, MODE_DIAG, USER>(d, wg, stage, par, sim0, tab, cached, nullptr, nullptr);
+    if (wg < ngroups) forces_group<T, L, S, ONE, MODE_DIAG, USER>(d, wg, stage, par, sim0, tab, cached, nullptr, nullptr, false);
 }
 
 // Stand-alone rebuild phases (update_neighbors!, and the stateless neighbour

@@ -199,7 +199,7 @@ const Variant VARIANTS[] = {
     {16, 3, 256, 2, step_fn<float, 16, 3, 256, 2>, nullptr, stage_bytes_per_warp<float, 16>(), 0, 2},
     {8, 5, 128, 5, step_fn<float, 8, 5, 128, 5>, nullptr, stage_bytes_per_warp<float, 8>(), 0, 3},
     {16, 3, 128, 5, step_fn<float, 16, 3, 128, 5>, nullptr, stage_bytes_per_warp<float, 16>(), 0, 2},
-    {8, 5, 224, 2, step_fn<float, 8, 5, 224, 2>, step_fn<double, 8, 5, 224, 1>, stage_bytes_per_warp<float, 8>(),
+    {8, 5, 224, 2, step_fn<float, 8, 5, 224, 2>, step_fn<double, 8, 5, 224, 2>, stage_bytes_per_warp<float, 8>(),
      stage_bytes_per_warp<double, 8>(), 0},
 };
 constexpr int NVARIANTS = sizeof(VARIANTS) / sizeof(VARIANTS[0]);
@@ -535,6 +535,23 @@ std::vector<T> mode_table(int nth) {
     return t;
 }
 
+// FP64: the contraction matrix M of fcc_forces64.cuh, row k = (cos 2 phi_k,
+// sin 2 phi_k, ..., cos 10 phi_k, sin 10 phi_k, 1, 0), zero rows beyond the contour.
+template <>
+std::vector<double> mode_table<double>(int nth) {
+    std::vector<double> t((size_t)(nth + M64_PAD) * M64_COLS, 0.0);
+    for (int k = 0; k < nth; ++k) {
+        double* e = t.data() + (size_t)k * M64_COLS;
+        for (int m = 0; m < KM; ++m) {
+            const double a = (double)(m + 2) * k * (2 * PI / nth);
+            e[2 * m] = std::cos(a);
+            e[2 * m + 1] = std::sin(a);
+        }
+        e[2 * KM] = 1.0;
+    }
+    return t;
+}
+
 // Round a float to TF32 (10 mantissa bits), to nearest with ties away from
 // zero: the rounding of cvt.rna.tf32.f32.
 float tf32_round(float x) {
@@ -819,11 +836,11 @@ struct Engine final : EngineBase {
 
     int variant = 0;
     const Variant& var() const { return VARIANTS[variant]; }
-    static constexpr size_t grad_stage_bytes() {
-        return basis_table_bytes<T>() + (size_t)(256 / 32) * stage_bytes_per_warp<T, LANES>();
+    static constexpr size_t grad_stage_bytes(bool one) {
+        return basis_table_bytes<T>(one) + (size_t)(256 / 32) * stage_bytes_per_warp<T, LANES>();
     }
     size_t stage_bytes() const {
-        return basis_table_bytes<T>() + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
+        return basis_table_bytes<T>(nth <= var().L * var().S) + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
     }
     // compiled user terms: the 8 x 5 / 256-thread kernels with the user-term code
     bool user = false;
@@ -901,7 +918,7 @@ struct Engine final : EngineBase {
         FCC_TRY(choose_variant());
         const int smem = (int)stage_bytes();
         CUDA_TRY(cudaFuncSetAttribute(step_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        CUDA_TRY(cudaFuncSetAttribute(grad_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_stage_bytes()));
+        CUDA_TRY(cudaFuncSetAttribute(grad_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grad_stage_bytes(nth <= LANES * SLOTS)));
         int per_sm = 0;
         const int blk = var().blk;
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, step_kernel(), blk, smem));
@@ -1122,11 +1139,11 @@ struct Engine final : EngineBase {
         const int64_t groups = (N + (32 / LANES) - 1) / (32 / LANES);
         const int grid = (int)((groups + 256 / 32 - 1) / (256 / 32));
         if (user)
-            k_gradients<T, LANES, SLOTS, true, true><<<grid, 256, grad_stage_bytes(), stream>>>(d, par());
+            k_gradients<T, LANES, SLOTS, true, true><<<grid, 256, grad_stage_bytes(nth <= LANES * SLOTS), stream>>>(d, par());
         else if (nth <= LANES * SLOTS)
-            k_gradients<T, LANES, SLOTS, true><<<grid, 256, grad_stage_bytes(), stream>>>(d, par());
+            k_gradients<T, LANES, SLOTS, true><<<grid, 256, grad_stage_bytes(nth <= LANES * SLOTS), stream>>>(d, par());
         else
-            k_gradients<T, LANES, SLOTS, false><<<grid, 256, grad_stage_bytes(), stream>>>(d, par());
+            k_gradients<T, LANES, SLOTS, false><<<grid, 256, grad_stage_bytes(nth <= LANES * SLOTS), stream>>>(d, par());
         CUDA_TRY(cudaGetLastError());
         return sync_stream();
     }

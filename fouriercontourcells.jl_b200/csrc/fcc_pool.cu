@@ -293,7 +293,7 @@ struct Pool final : PoolBase {
     bool split() const { return nsplit > 0; }
     void* step_kernel() const { return (sizeof(T) == 4 ? var().f32 : var().f64)(nth <= var().L * var().S, split()); }
     size_t stage_bytes() const {
-        return basis_table_bytes<T>() + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
+        return basis_table_bytes<T>(nth <= var().L * var().S) + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
     }
 
     fcc_status init(const fcc_pool_params& q) {
