@@ -67,7 +67,8 @@ __device__ __forceinline__ void update_body64(const DevPtrs<double>& d, const Si
                                               int l, int par, double xo, double yo, double wo, double tho, double r0,
                                               int ti, double fx, double fy, double tt, double gl0, const double (&gA)[2],
                                               const double (&gB)[2], const double* scf, double x0, double y0,
-                                              double rmax0, int fl, const double (&nz)[2], int* rbp) {
+                                              double rmax0, int fl, const double (&nz)[2], int* rbp, double* own,
+                                              double* scf_w, bool keep) {
     typedef double T;
     constexpr int L = 8;
     constexpr unsigned FULL = 0xffffffffu;
@@ -172,6 +173,12 @@ __device__ __forceinline__ void update_body64(const DevPtrs<double>& d, const Si
                 rn[r_be(m)] = r0 * be;
                 cf[1 + m] = an[u];
                 cf[1 + KM + m] = bn[u];
+                if (keep) {
+                    own[r_al(m)] = r0 * al;
+                    own[r_be(m)] = r0 * be;
+                    scf_w[1 + m] = an[u];
+                    scf_w[1 + KM + m] = bn[u];
+                }
             }
         }
     }
@@ -187,6 +194,17 @@ __device__ __forceinline__ void update_body64(const DevPtrs<double>& d, const Si
         rn[R_A0] = r0 * a0n;
         rn[R_TH] = thn;
         cf[0] = a0n;
+        if (keep) {  // where the next step reads them (Resident)
+            own[R_X] = xw;
+            own[R_Y] = yw;
+            own[R_RMAX] = rmax;
+            own[R_A0] = r0 * a0n;
+            own[R_TH] = thn;
+            scf_w[0] = a0n;
+            scf_w[NCM] = sn1;
+            scf_w[NCM + 1] = cn1;
+            scf_w[NCM + 2] = T(0.5) / a0n;
+        }
         // skin check of the new state (src/neighbors.jl:198-205); the flags of
         // this step (read at its start) already carry F_VALID of a rebuild
         if ((fl & F_CONTACT) && (fl & F_VALID) && P.skin > T(0)) {
@@ -201,18 +219,13 @@ __device__ __forceinline__ void update_body64(const DevPtrs<double>& d, const Si
     }
 }
 
-template <bool V>
-struct Flag {
-    static constexpr bool value = V;
-};
-
 // Forces on the 4 bodies of warp group `wg`, and in MODE_FUSED their update
 // (references: forces_warp).  `stage` is this warp's shared memory; `tab` the
 // block's copy of M and of the nodes' (cos, sin) (one chunk), else null.
-template <bool ONE, int MODE, bool USER>
+template <bool ONE, int MODE, bool USER, bool LAT>
 __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, double* stage, int par,
                                               const SimDesc<double>* sim0, const double* tab, int* rbp,
-                                              const BarrierLocal* lone, bool drawn) {
+                                              const BarrierLocal* lone, bool drawn, Resident<double, 8>* res) {
     typedef double T;
     constexpr int L = 8, S = 5, BPW = 4;
     constexpr unsigned FULL = 0xffffffffu;
@@ -248,23 +261,38 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
 
     // ---- independent loads first
     const T* grec = rc + (size_t)gg * RECW;
-    for (int c = l; c < RECW / 2; c += L) cp_async16(own + 2 * c, grec + 2 * c);
-    if (MODE != MODE_FORCES) {
-        const T* cf = d.coef + (size_t)gg * NCM;  // written by this block only (during a launch)
+    T xi, yi, rmi, wf, r0;
+    const bool kept = LAT && res->have;
+    if (kept) {  // the own state is where the last update left it
+        xi = own[R_X], yi = own[R_Y], wf = own[R_W];
+        r0 = res->r0;
+    } else {
+        for (int c = l; c < RECW / 2; c += L) cp_async16(own + 2 * c, grec + 2 * c);
+        if (MODE != MODE_FORCES) {
+            const T* cf = d.coef + (size_t)gg * NCM;  // written by this block only (during a launch)
 #pragma unroll
-        for (int u = 0; u < 3; ++u)
-            if (l + u * L < NCM) cp_async8(scf + l + u * L, cf + l + u * L);
+            for (int u = 0; u < 3; ++u)
+                if (l + u * L < NCM) cp_async8(scf + l + u * L, cf + l + u * L);
+        }
+        load_head(grec, xi, yi, rmi, wf);
+        r0 = __ldg(d.R0 + gg);
     }
     cp_async_commit();
-    T xi, yi, rmi, wf;
-    load_head(grec, xi, yi, rmi, wf);
-    const T r0 = __ldg(d.R0 + gg);
-    const int cnt_raw = ldcg(d.nb_count + gg);
-    int ids[IDS];
-#pragma unroll
-    for (int u = 0; u < IDS; ++u) {
-        const int q = l + u * L;
-        ids[u] = q < min(d.cap, NBMAX64) ? ldcg(d.nb_idx + (size_t)gg * d.cap + q) : gg;
+    int cnt_raw, ids[IDS];
+    static_assert(IDS == 1, "one neighbour id per lane");
+    if (kept && res->lists) {
+        cnt_raw = res->cnt;
+        ids[0] = res->ids[0];
+    } else {
+        cnt_raw = ldcg(d.nb_count + gg);
+        ids[0] = l < min(d.cap, NBMAX64) ? ldcg(d.nb_idx + (size_t)gg * d.cap + l) : gg;
+    }
+    const bool ref = kept && res->lists;  // the skin references of the last rebuild are at hand
+    if constexpr (LAT) {
+        res->r0 = r0;
+        res->cnt = cnt_raw;
+        res->ids[0] = ids[0];
+        res->lists = true;
     }
     const int fl = lone ? lone->flags : ldcg(d.flags + s);
     const long long clk = lone ? lone->clock : ldcg(d.clock + s);
@@ -294,7 +322,7 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
     const T Lx = P.Lx, Ly = P.Ly;
     const T cB = P.cB[ti];
     auto stage_batch = [&](int base, bool have) {  // have: ids holds the batch's ids
-        const int npre = min(cnt - base, NBMAX64), most = min(maxc - base, NBMAX64);
+        const int npre = min(cnt - base, NBMAX64);
         __syncwarp();
         if (!have) {
 #pragma unroll
@@ -303,16 +331,16 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
                 ids[u] = q < npre ? ldcg(d.nb_idx + (size_t)gg * d.cap + base + q) : gg;
             }
         }
+        int j[NBMAX64];
 #pragma unroll
-        for (int q = 0; q < NBMAX64; ++q) {
-            if (q >= most) break;
-            const int j = __shfl_sync(FULL, ids[q / L], q % L, L);
+        for (int q = 0; q < NBMAX64; ++q) j[q] = __shfl_sync(FULL, ids[q / L], q % L, L);
+#pragma unroll
+        for (int q = 0; q < NBMAX64; ++q)
             if (q < npre) {
-                const T* src = rc + (size_t)j * RECW;
+                const T* src = rc + (size_t)j[q] * RECW;
                 cp_async16(snb + q * SREC64 + 2 * l, src + 2 * l);
                 if (l < RECW / 2 - L) cp_async16(snb + q * SREC64 + 2 * (l + L), src + 2 * (l + L));
             }
-        }
         cp_async_commit();
     };
     auto finish_batch = [&](int base) {
@@ -426,7 +454,7 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
     }
 
     // what the update needs of the own state alone, while the neighbours' copies arrive
-    if (MODE == MODE_FUSED && l == 0) {
+    if (MODE == MODE_FUSED && !kept && l == 0) {
         T so, co;
         t_sincos(own[R_TH], &so, &co);
         scf[NCM] = so;
@@ -594,8 +622,15 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
         }
     }
     // skin reference of the update: under way during the sums
-    const T x0 = MODE == MODE_FUSED ? ldcg(d.x0 + gg) : T(0), y0 = MODE == MODE_FUSED ? ldcg(d.y0 + gg) : T(0),
-            rmax0 = MODE == MODE_FUSED ? ldcg(d.rmax0 + gg) : T(0);
+    T x0 = T(0), y0 = T(0), rmax0 = T(0);
+    if (LAT && ref) {
+        x0 = res->pre.x0, y0 = res->pre.y0, rmax0 = res->pre.rmax0;
+    } else if (MODE == MODE_FUSED) {
+        x0 = ldcg(d.x0 + gg);
+        y0 = ldcg(d.y0 + gg);
+        rmax0 = ldcg(d.rmax0 + gg);
+        if constexpr (LAT) res->pre.x0 = x0, res->pre.y0 = y0, res->pre.rmax0 = rmax0;
+    }
     // ---- mode gradients of the lab frame (/ R0): lane l has those of mode l,
     // lane 0 those of mode 8 too; dE/da0 to every lane of the body
     T gA[MPL], gB[MPL], gl0;
@@ -668,7 +703,7 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
     }
     if (valid && !act) carry_record_staged<T, L>(d, g, l, par, own);
     update_body64(d, P, act, g, s, l, par, xi, yi, wf, own[R_TH], r0, ti, fx, fy, tt, gl0, gA, gB, scf, x0, y0, rmax0, fl,
-                  nz, rbp);
+                  nz, rbp, own, scf, LAT && res->on);
 }
 
 }  // namespace fcc

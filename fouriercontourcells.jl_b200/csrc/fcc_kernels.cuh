@@ -925,6 +925,20 @@ __device__ __forceinline__ void load_update_pre(const DevPtrs<T>& d, int gg, int
     }
 }
 
+// What a warp keeps of its bodies from one step to the next in a launch whose
+// blocks hold at most one warp group per warp (k_step's LAT kernels, one
+// simulation): the own records stay in its shared memory, the rest here, so a
+// step reads only the neighbours' records from L2.  `lists`: the neighbour
+// ids, counts and skin references are those of the last rebuild.
+template <class T, int L>
+struct Resident {
+    bool on, have, lists;
+    int ids[(16 + L - 1) / L];
+    int cnt;
+    T r0, so, co;  // radius scale, sin and cos of theta
+    UpdatePre<T, L> pre;
+};
+
 // (cos n t, sin n t) from (cos t, sin t) by binary powering, n = 2..10 (a
 // few complex products instead of one sincos per mode).
 // Per-mode pieces of the end of a step, shared by the update and by k_init so
@@ -1035,16 +1049,16 @@ __device__ __forceinline__ void lane_mode_grads(const T (&gl)[NCM], int l, T (&g
 // lab frame of the new state into rec[next], skin check.  fx, fy, tt and gl0
 // (dE/da0 of the lab frame / R0) are uniform across the group; gA, gB are the
 // lab-frame mode gradients of the lane's modes (lane_mode_grads).
-template <class T, int L>
+template <class T, int L, bool LAT = false>
 __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T>& P, bool act, int g, int s, int l,
                                             int par, long long clk, T xo, T yo, T wo, T tho, T r0, int ti, T fx, T fy,
                                             T tt, T gl0, const T (&gA)[UpdatePre<T, L>::MPL],
                                             const T (&gB)[UpdatePre<T, L>::MPL], const UpdatePre<T, L>& pre, int fl,
-                                            const T (&nz)[2], bool split, int* rbp) {
+                                            const T (&nz)[2], bool split, int* rbp, T* own = nullptr,
+                                            Resident<T, L>* res = nullptr) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int MPL = UpdatePre<T, L>::MPL;
     const T dt = P.dt;
-    const uint32_t li = (uint32_t)(g - P.body_off + 1);
     // standard normals of this body and step (src/random.jl:88-100): lane 0
     // holds block 1 (orientation), lane 1 block 0 (translation)
     const T z3 = __shfl_sync(FULL, nz[0], 0, L);
@@ -1053,7 +1067,8 @@ __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T
     const T sig_r = P.sigr[ti];
     const T thn = tho - (dt * P.muth[ti]) * tt + sig_r * z3;
     T so1, co1, sn1, cn1;
-    t_sincos(tho, &so1, &co1);
+    if (LAT && res->have) so1 = res->so, co1 = res->co;
+    else t_sincos(tho, &so1, &co1);
     t_sincos(thn, &sn1, &cn1);
 
     T* cf = d.coef + (size_t)(act ? g : 0) * NCM;
@@ -1132,8 +1147,19 @@ __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T
                 rn[r_be(m)] = r0 * be;
                 cf[1 + m] = an[u];
                 cf[1 + KM + m] = bn[u];
+                if (LAT && res->on) {
+                    own[r_al(m)] = r0 * al;
+                    own[r_be(m)] = r0 * be;
+                    res->pre.a[u] = an[u];
+                    res->pre.b[u] = bn[u];
+                }
             }
         }
+    }
+    if (LAT) {
+        res->so = act ? sn1 : so1;
+        res->co = act ? cn1 : co1;
+        if (act) res->pre.a0 = a0n;
     }
     const T rmax = r0 * (a0n + bp);
 
@@ -1168,6 +1194,13 @@ __device__ __forceinline__ void update_body(const DevPtrs<T>& d, const SimDesc<T
         rn[R_A0] = r0 * a0n;
         rn[R_TH] = thn;
         cf[0] = a0n;
+        if (LAT && res->on) {
+            own[R_X] = xw;
+            own[R_Y] = yw;
+            own[R_RMAX] = rmax;
+            own[R_A0] = r0 * a0n;
+            own[R_TH] = thn;
+        }
         // skin check of the new state (src/neighbors.jl:198-205); the flags of
         // this step (read at its start) already carry F_VALID of a rebuild
         if ((fl & F_CONTACT) && (fl & F_VALID) && P.skin > T(0)) {
@@ -1202,6 +1235,11 @@ __device__ __forceinline__ void carry_record_staged(const DevPtrs<T>& d, int g, 
 
 // ==================================================== force evaluation ==
 enum : int { MODE_FUSED = 0, MODE_FORCES = 1, MODE_DIAG = 2 };
+
+template <bool V>
+struct Flag {
+    static constexpr bool value = V;
+};
 
 // Body terms of the contour integral Q: W = sum_t dF_t/dQ * dphi, the energy
 // E = e_1 + (e_2 + ...) (src/energies/body_terms.jl:8-34).
@@ -1370,6 +1408,80 @@ __device__ __forceinline__ void bond_forces(const DevPtrs<T>& d, const SimDesc<T
 
 namespace fcc {
 
+// Contact phases of the LAT kernels on neighbours q0 .. q1 - 1 of a staged
+// batch (heads as finish_batch leaves them; n: the body's records in it): the
+// same tests, values and order of sums as in forces_warp, with two hits of a
+// lane in flight.  With one warp group per warp nothing else hides a hit's
+// chain of some 300 cycles; with more (the other kernels) the second hit's
+// work costs more than it hides (N = 16384: 24.5 against 24.3 us a step).
+template <class T, int S>
+__device__ __forceinline__ void contact_lat(const T* snb, int n, int q0, int q1, const T (&R)[S], const T (&C1)[S],
+                                            const T (&S1)[S], unsigned vmask, bool rewrap, T Lx, T Ly, T iLx, T iLy,
+                                            T cB, T* wsl) {
+    unsigned long long hm = 0;
+    const int qe = min(q1, n);
+    auto test = [&](auto wrap) {
+#pragma unroll 2
+        for (int qq = q0; qq < qe; ++qq) {
+            T ox, oy, lim2, cA;
+            lds_head(snb + qq * RECW, ox, oy, lim2, cA);
+            unsigned m = 0;
+#pragma unroll
+            for (int sl = 0; sl < S; ++sl) {
+                T dx = R[sl] * C1[sl] + ox, dy = R[sl] * S1[sl] + oy;
+                if constexpr (decltype(wrap)::value) {
+                    dx = minimum_image_fast(dx, Lx, iLx);
+                    dy = minimum_image_fast(dy, Ly, iLy);
+                }
+                m |= (dx * dx + dy * dy <= lim2) ? (1u << sl) : 0u;
+            }
+            hm |= (unsigned long long)(m & vmask) << ((qq - q0) * S);
+        }
+    };
+    if (rewrap) test(Flag<true>{});
+    else test(Flag<false>{});
+    while (hm) {
+        int bit[2], sl[2];
+        const T* r[2];
+        T dx[2], dy[2], gv[2], cA[2];
+        bit[0] = __ffsll((long long)hm) - 1;
+        hm &= hm - 1;
+        const bool two = hm != 0;
+        bit[1] = two ? __ffsll((long long)hm) - 1 : bit[0];
+        hm &= hm - 1;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            sl[i] = bit[i] - (bit[i] / S) * S;
+            r[i] = snb + (q0 + bit[i] / S) * RECW;
+            T ox, oy, lim2;
+            lds_head(r[i], ox, oy, lim2, cA[i]);
+            const auto e = lds4(wsl + sl[i] * 4);
+            dx[i] = e.x * e.y + ox;
+            dy[i] = e.x * e.z + oy;
+        }
+        if (rewrap) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                dx[i] = minimum_image_fast(dx[i], Lx, iLx);
+                dy[i] = minimum_image_fast(dy[i], Ly, iLy);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const T d2 = dx[i] * dx[i] + dy[i] * dy[i];
+            const bool off = d2 > T(0);
+            T dist, inv;
+            norm_inv(d2, dist, inv);
+            const T cp = off ? dx[i] * inv : T(1), sp = off ? dy[i] * inv : T(0);
+            const T dd = radius_at(r[i], cp, sp) - (off ? dist : T(0));
+            gv[i] = dd >= T(0) ? cA[i] : T(0);
+            gv[i] = dd > T(0) ? gv[i] + cB * dd : gv[i];
+        }
+        wsl[sl[0] * 4 + 3] += gv[0];
+        if (two) wsl[sl[1] * 4 + 3] += gv[1];
+    }
+}
+
 // Forces on the 32/L bodies of warp group `wg`, and in MODE_FUSED their
 // update.  `stage` is this warp's shared-memory slot for neighbour records.
 // Follows, per body i:
@@ -1382,9 +1494,9 @@ namespace fcc {
 // USER: the simulation has compiled user terms (include/fcc_user_terms.h):
 // R'' is synthesised, user integrals, node gradients (GDD included),
 // pressures and bond gradients are added, and the pullback includes R''.
-template <class T, int L, int S, bool ONE, int MODE, bool USER = false>
+template <class T, int L, int S, bool ONE, int MODE, bool USER = false, bool LAT = false>
 __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stage, int par, const SimDesc<T>* sim0,
-                                            const T* tab, int& cached, int* rbp, const BarrierLocal* lone, bool drawn) {
+                                            const T* tab, int& cached, int* rbp, const BarrierLocal* lone, bool drawn, Resident<T, L>* res = nullptr) {
     constexpr int BPW = 32 / L;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int CH16 = RECW * (int)sizeof(T) / 16;  // 16-byte chunks per record
@@ -1429,24 +1541,53 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     T* own = stage + (size_t)(lane / L) * RECW;
     T* snb = stage + (size_t)BPW * RECW + (size_t)(lane / L) * NBMAX * RECW;
     const T* grec = rc + (size_t)gg * RECW;
-    T xi, yi, rmi, wf;
-    load_head(grec, xi, yi, rmi, wf);
-    const T a0r = ldcg(grec + R_A0), th = ldcg(grec + R_TH);
-    for (int c = l; c < CH16; c += L) cp_async16(own + c * (16 / sizeof(T)), grec + c * (16 / sizeof(T)));
-    cp_async_commit();
-    const T r0 = __ldg(d.R0 + gg);
-    const int cnt_raw = ldcg(d.nb_count + gg);
+    T xi, yi, rmi, wf, a0r, th, r0;
+    int cnt_raw;
     int ids[IDS];
+    const bool kept = LAT && res->have;
+    if (kept) {  // the own record is where the last update left it
+        lds_head(own, xi, yi, rmi, wf);
+        a0r = own[R_A0];
+        th = own[R_TH];
+        r0 = res->r0;
+    } else {
+        load_head(grec, xi, yi, rmi, wf);
+        a0r = ldcg(grec + R_A0), th = ldcg(grec + R_TH);
+        for (int c = l; c < CH16; c += L) cp_async16(own + c * (16 / sizeof(T)), grec + c * (16 / sizeof(T)));
+        r0 = __ldg(d.R0 + gg);
+    }
+    cp_async_commit();
+    if (kept && res->lists) {
+        cnt_raw = res->cnt;
 #pragma unroll
-    for (int u = 0; u < IDS; ++u) {
-        const int q = l + u * L;
-        ids[u] = q < min(d.cap, NBMAX) ? ldcg(d.nb_idx + (size_t)gg * d.cap + q) : gg;
+        for (int u = 0; u < IDS; ++u) ids[u] = res->ids[u];
+    } else {
+        cnt_raw = ldcg(d.nb_count + gg);
+#pragma unroll
+        for (int u = 0; u < IDS; ++u) {
+            const int q = l + u * L;
+            ids[u] = q < min(d.cap, NBMAX) ? ldcg(d.nb_idx + (size_t)gg * d.cap + q) : gg;
+        }
     }
     // a lone simulation's flags and clock are known to the block (released with the barrier)
     const int fl = lone ? lone->flags : ldcg(d.flags + s);
     const long long clk = lone ? lone->clock : ldcg(d.clock + s);
     UpdatePre<T, L> pre;
-    if (MODE == MODE_FUSED) load_update_pre(d, gg, l, P.K, pre);
+    if (MODE == MODE_FUSED) {
+        if (kept && res->lists) {
+            pre = res->pre;
+        } else {
+            load_update_pre(d, gg, l, P.K, pre);
+        }
+    }
+    if constexpr (LAT) {
+        res->r0 = r0;
+        res->cnt = cnt_raw;
+#pragma unroll
+        for (int u = 0; u < IDS; ++u) res->ids[u] = ids[u];
+        res->pre = pre;
+        res->lists = true;
+    }
     bool act = valid;
     if (MODE != MODE_DIAG) act = act && (fl & F_ACTIVE) && !(fl & (F_FROZEN | F_HOLD));
     const int nth = P.nth;
@@ -1466,9 +1607,24 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     // ---- stage the neighbour records in shared memory (cp.async)
     const bool contact = act && (fl & F_CONTACT);
     const int cnt = contact ? min(cnt_raw, d.cap) : 0;
-    auto stage_batch = [&](int base) {
+    const int maxc = __reduce_max_sync(FULL, cnt);
+    auto stage_batch = [&](int base, bool have) {  // have: ids holds the batch's ids
         const int npre = min(cnt - base, NBMAX);
         __syncwarp();  // every lane is done with the previous contents
+        if constexpr (LAT) {  // a record by the lanes of its body
+#pragma unroll
+            for (int u = 0; u < IDS; ++u)
+                if (!have && l + u * L < npre) ids[u] = ldcg(d.nb_idx + (size_t)gg * d.cap + base + l + u * L);
+            int j[NBMAX];
+#pragma unroll
+            for (int q = 0; q < NBMAX; ++q) j[q] = __shfl_sync(FULL, ids[q / L], q % L, L);
+#pragma unroll
+            for (int q = 0; q < NBMAX; ++q)
+                if (q < npre && l < CH16)
+                    cp_async16(snb + q * RECW + l * (16 / sizeof(T)), rc + (size_t)j[q] * RECW + l * (16 / sizeof(T)));
+            cp_async_commit();
+            return;
+        }
 #pragma unroll
         for (int u = 0; u < IDS; ++u) {
             const int q = l + u * L;
@@ -1481,12 +1637,38 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         }
         cp_async_commit();
     };
-    stage_batch(0);
-    int staged_base = 0;
-
     const int wv = unpack_w(wf);
     const int ti = wv & 7;
     const int pi = wv >> 3;
+    // LAT: a batch once it has arrived: lane q replaces the head of record q by
+    // the minimum-image centre offset r_i - r_j, the squared reach and the
+    // pair's coupling, which the contact phases then read
+    auto finish_batch = [&](int base) {
+        cp_async_wait_all();
+        __syncwarp();
+        if constexpr (LAT) {
+            const int npre = min(cnt - base, NBMAX);
+#pragma unroll
+            for (int u = 0; u < IDS; ++u) {
+                const int q = l + u * L;
+                if (q < npre) {
+                    T* r = snb + q * RECW;
+                    T xj, yj, rmj, wj;
+                    lds_head(r, xj, yj, rmj, wj);
+                    const int wjv = unpack_w(wj);
+                    const T lim = rmj + P.crange;
+                    r[R_X] = minimum_image_fast(xi - xj, P.Lx, P.invLx);
+                    r[R_Y] = minimum_image_fast(yi - yj, P.Ly, P.invLy);
+                    r[R_RMAX] = lim * lim;
+                    r[R_W] = P.cA[(wjv >> 3) == pi ? 1 : 0][ti][wjv & 7];
+                }
+            }
+            __syncwarp();
+        }
+    };
+    stage_batch(0, true);
+    int staged_base = 0;
+
 
     T R[S], R1[S], C1[S], S1[S];
     T R2[S];  // R'' (user terms only)
@@ -1630,9 +1812,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         for (int r = 0; r < NCM; ++r) gl[r] = T(0);
     }
 
-    cp_async_wait_all();
-    __syncwarp();
-    const int maxc = __reduce_max_sync(FULL, cnt);
+    finish_batch(0);
     const T Lx = P.Lx, Ly = P.Ly, iLx = P.invLx, iLy = P.invLy, crange = P.crange;
     const bool rewrap = P.rewrap != 0;
 
@@ -1659,9 +1839,8 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
             constexpr int QB = 64 / S;  // neighbours per 64-bit hit mask
             for (int base = 0; base < maxc; base += NBMAX) {
                 if (base != staged_base) {  // lists longer than the stage: restage
-                    stage_batch(base);
-                    cp_async_wait_all();
-                    __syncwarp();
+                    stage_batch(base, false);
+                    finish_batch(base);
                     staged_base = base;
                 }
                 const int qn = min(maxc - base, NBMAX);
@@ -1670,6 +1849,10 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
                     // neighbour: bit (q - q0) * S + slot of a 64-bit hit mask
                     unsigned long long hm = 0;
                     const int q1 = min(qn, q0 + QB);
+                    if constexpr (LAT) {
+                        contact_lat<T, S>(snb, cnt - base, q0, q1, R, C1, S1, vmask, rewrap, Lx, Ly, iLx, iLy, P.cB[ti], wsl);
+                        continue;
+                    }
                     for (int qq = q0; qq < q1; ++qq) {
                         if (base + qq < cnt) {
                             T xj, yj, rmj, wj;
@@ -1959,17 +2142,17 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         d.E[g] = E;
     }
     if (valid && !act) carry_record_staged<T, L>(d, g, l, par, own);
-    update_body<T, L>(d, P, act, g, s, l, par, clk, xi, yi, wf, th, r0, ti, fx, fy, tt, gl0, gA, gB, pre, fl, nz, false,
-                      rbp);
+    update_body<T, L, LAT>(d, P, act, g, s, l, par, clk, xi, yi, wf, th, r0, ti, fx, fy, tt, gl0, gA, gB, pre, fl, nz,
+                           false, rbp, own, res);
 }
 
 // The force evaluation of a precision.
-template <class T, int L, int S, bool ONE, int MODE, bool USER>
+template <class T, int L, int S, bool ONE, int MODE, bool USER, bool LAT>
 __device__ __forceinline__ void forces_group(const DevPtrs<T>& d, int wg, T* stage, int par, const SimDesc<T>* sim0,
                                              const T* tab, int& cached, int* rbp, const BarrierLocal* lone,
-                                             bool drawn) {
-    if constexpr (sizeof(T) == 8) forces_warp64<ONE, MODE, USER>(d, wg, stage, par, sim0, tab, rbp, lone, drawn);
-    else forces_warp<T, L, S, ONE, MODE, USER>(d, wg, stage, par, sim0, tab, cached, rbp, lone, drawn);
+                                             bool drawn, Resident<T, L>* res) {
+    if constexpr (sizeof(T) == 8) forces_warp64<ONE, MODE, USER, LAT>(d, wg, stage, par, sim0, tab, rbp, lone, drawn, res);
+    else forces_warp<T, L, S, ONE, MODE, USER, LAT>(d, wg, stage, par, sim0, tab, cached, rbp, lone, drawn, res);
 }
 
 // Normals of warp group wg's bodies in draw clk of a lone simulation, left in
@@ -2223,6 +2406,7 @@ __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
 // each warp its first and then the block's next untaken one.
 template <class T, int L, int S, bool ONE, bool SPLIT, int BLK, int MINB, bool USER = false>
 __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, int par0) {
+    constexpr bool LAT = MINB == 1 && ONE && !SPLIT && L == 8 && S == 5;
     const int WPB = blockDim.x >> 5;  // at most BLK / 32
     const int warp = threadIdx.x >> 5;
     const int ngroups = (d.Ntot + (32 / L) - 1) / (32 / L);
@@ -2250,6 +2434,11 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
     // next step while they wait at the step barrier
     const bool ahead = FCC_FLAT_BARRIER && !SPLIT && !USER && lone && sim0->has_noise;
     bool drawn = false;
+    // One block of registers per SM (MINB = 1): the kernels for grids that hold
+    // at most one warp group per warp, where a group's chain of latencies is
+    // the step.  There a warp keeps its bodies' state from step to step.
+    Resident<T, L> res{};
+    res.on = LAT && lone && g1 - g0 <= WPB;
     for (int st = 0; st < nsteps; ++st) {
         const int par = (par0 + st) & 1;
         if (bl.any) {
@@ -2259,27 +2448,29 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
                                   (int)(WPB * stage_bytes_per_warp<T, L>() / sizeof(int))))
                 return;
             cached = -1;  // the descriptor slots were overwritten
+            res.lists = false;
         }
         if (dyn) {
             // a warp's first group is its own; after that it takes the block's
             // next untaken group (groups cost unequal time: contacts, hits)
             if (threadIdx.x == 0) s_next[(st + 1) & 1] = g0 + WPB;  // last used by the previous step
             for (int wg = g0 + warp; wg < g1;) {
-                forces_group<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER>(d, wg, stage, par, sim0, tab,
+                forces_group<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER, LAT>(d, wg, stage, par, sim0, tab,
                                                                                    cached, &bl.rebuild,
                                                                                    lone ? &bl : nullptr,
-                                                                                   drawn && wg == g0 + warp);
+                                                                                   drawn && wg == g0 + warp, &res);
                 int nx = 0;
                 if ((threadIdx.x & 31) == 0) nx = atomicAdd(&s_next[st & 1], 1);
                 wg = __shfl_sync(0xffffffffu, nx, 0);
             }
         } else {
             for (int wg = g0 + warp; wg < g1; wg += WPB)
-                forces_group<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER>(d, wg, stage, par, sim0, tab,
+                forces_group<T, L, S, ONE, SPLIT ? MODE_FORCES : MODE_FUSED, USER, LAT>(d, wg, stage, par, sim0, tab,
                                                                                    cached, &bl.rebuild,
                                                                                    lone ? &bl : nullptr,
-                                                                                   drawn && wg == g0 + warp);
+                                                                                   drawn && wg == g0 + warp, &res);
         }
+        if (LAT) res.have = res.on;
         if (SPLIT) {
             if (!grid_barrier(d.sync, bl, [](unsigned) { return -1; })) return;
             for (int wg = g0 + warp; wg < g1; wg += WPB) update_warp_split<T, L>(d, wg, par, sim0, &bl.rebuild);
@@ -2352,7 +2543,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_gradients(DevPt
     const T* tab = stage_basis<T, ONE>(d);
     const SimDesc<T>* sim0 = copy_desc(d);
     int cached = -1;
-    if (wg < ngroups) forces_group<T, L, S, ONE, MODE_DIAG, USER>(d, wg, stage, par, sim0, tab, cached, nullptr, nullptr, false);
+    if (wg < ngroups)
+        forces_group<T, L, S, ONE, MODE_DIAG, USER, false>(d, wg, stage, par, sim0, tab, cached, nullptr, nullptr, false,
+                                                           nullptr);
 }
 
 // Stand-alone rebuild phases (update_neighbors!, and the stateless neighbour

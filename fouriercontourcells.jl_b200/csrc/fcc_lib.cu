@@ -201,6 +201,7 @@ const Variant VARIANTS[] = {
     {16, 3, 128, 5, step_fn<float, 16, 3, 128, 5>, nullptr, stage_bytes_per_warp<float, 16>(), 0, 2},
     {8, 5, 224, 2, step_fn<float, 8, 5, 224, 2>, step_fn<double, 8, 5, 224, 2>, stage_bytes_per_warp<float, 8>(),
      stage_bytes_per_warp<double, 8>(), 0},
+    {8, 5, 256, 1, step_fn<float, 8, 5, 256, 1>, nullptr, stage_bytes_per_warp<float, 8>(), 0, 0},
 };
 constexpr int NVARIANTS = sizeof(VARIANTS) / sizeof(VARIANTS[0]);
 constexpr int LANES = 8, SLOTS = 5;  // compute_gradients and the FP64 step
@@ -642,7 +643,7 @@ struct Engine final : EngineBase {
     int64_t builds_adjust = 0;
     double last_ms = 0;
     int64_t last_launches = 0, last_steps = 0;
-    int step_grid = 0;
+    int step_grid = 0, step_blk = 0;  // launch shape of the step kernel
     // device buffers
     DBuf<SimDesc<T>> sims;
     DBuf<T> rec0, rec1, coef, R0, x0, y0, rmax0, cs, basis, gx, gy, gth, glab, E, P, GR, GD, GDD, gcoef;
@@ -859,20 +860,25 @@ struct Engine final : EngineBase {
     bool one_chunk() const { return nth <= var().L * var().S; }
 
     // Variant choice.  FCC_VARIANT overrides (FP64: only variants with an FP64
-    // build).  Otherwise a one-chunk step without parent drag compares the
-    // launch shapes of the default family (bit-identical results, FP32 and
-    // FP64) by the rounds of warp groups a step takes at this N, weighted by
-    // the measured time of one round.  224-thread blocks (14 warps per SM in
-    // FP32, 7 in FP64) run a round in about 0.97 (FP32) or 0.945 (FP64) of the
-    // time of 256-thread blocks but hold 12.5% fewer warps.  FP32 takes its
-    // groups dynamically, so a step costs whole rounds: 224 wins where the
-    // 256-thread grid leaves its last round part-empty (N = 1024: 9.57 vs
-    // 10.03 µs; N = 16384: 23.44 vs 23.45 µs, 61.4 vs 65.4 µs with a rebuild
-    // every step) and loses where both fill it (N = 65536: 88.1 vs 78.6 µs).
-    // FP64 splits them statically, so a step costs the mean rounds per warp
-    // (at least one): 224 wins only while one round holds all groups (N =
-    // 1024: 16.4 vs 16.6 µs; N = 16384: 63.1 vs 60.3 µs).  (Deformed states
-    // after 300 warm-up steps, flat step barrier.)
+    // build).  Otherwise a one-chunk step without parent drag chooses among
+    // the launch shapes of the default family (bit-identical results, FP32 and
+    // FP64) by the warp groups of this N:
+    //   - groups that fit one round of 8 warps per SM (N <= 4736 on 148 SMs):
+    //     the kernels built for latency (one block of registers per SM; FP32
+    //     variant 6, FP64 variant 0).  us a step (before, other shapes / this):
+    //     FP32 N = 1024 9.08 / 8.00, 4096 9.20 / 8.40; FP64 10.6 / 8.3 and
+    //     10.8 / 9.5.  In two rounds they lose: N = 6400 12.4 / 16.1, 15.1 / 17.1.
+    //   - more in FP64: 224-thread blocks, two per SM (variant 5; N = 6400
+    //     15.1 us against 17.1 with one block of 8 warps, 16384 28.2 / 34.0,
+    //     32580 56.2 / 60.2).
+    //   - more in FP32: 224- or 256-thread blocks, two per SM, by the rounds of
+    //     warp groups a step takes, weighted by the measured time of one round
+    //     (224-thread blocks 0.97 of 256-thread ones, with 12.5% fewer warps):
+    //     224 wins where the 256-thread grid leaves its last round part-empty
+    //     (N = 8280: 12.5 / 13.1 us; 16384: 22.7 / 23.1) and loses where both
+    //     fill it (65536: 88.1 / 78.6).
+    // Contours of several chunks and parent drag keep the base shape: FP64
+    // variant 0, and 5 once a round of variant 0 does not hold the groups.
     fcc_status choose_variant() {
         variant = 0;
         if (user) {  // one kernel family carries the user-term code
@@ -884,12 +890,22 @@ struct Engine final : EngineBase {
             if (v >= 0 && v < NVARIANTS && (sizeof(T) == 4 || VARIANTS[v].f64)) variant = v;
             return FCC_OK;
         }
-        if (N <= 0 || !one_chunk() || split) return FCC_OK;
+        if (N <= 0) return FCC_OK;
+        const bool one_round = (N + 3) / 4 <= (int64_t)nsm * 8;
+        if (sizeof(T) == 8) {
+            variant = one_round ? 0 : 5;
+            return FCC_OK;
+        }
+        if (!one_chunk() || split) return FCC_OK;
+        if (one_round) {
+            variant = 6;
+            return FCC_OK;
+        }
         struct Candidate {
             int v;
             double round_time;
         };
-        const Candidate cands[] = {{0, 1.0}, {5, sizeof(T) == 4 ? 0.97 : 0.945}};
+        const Candidate cands[] = {{0, 1.0}, {5, 0.97}};
         double best = 1e300;
         int pick = 0;
         for (const Candidate& c : cands) {
@@ -902,8 +918,7 @@ struct Engine final : EngineBase {
             const int64_t bpw = 32 / var().L, wpb = var().blk / 32;
             const int64_t groups = (N + bpw - 1) / bpw;
             const int64_t blocks = std::min<int64_t>((groups + wpb - 1) / wpb, (int64_t)per_sm * nsm);
-            const double rounds = sizeof(T) == 4 ? (double)((groups + blocks * wpb - 1) / (blocks * wpb))
-                                                 : std::max(1.0, (double)groups / (double)(blocks * wpb));
+            const double rounds = (double)((groups + blocks * wpb - 1) / (blocks * wpb));
             const double cost = rounds * c.round_time;
             if (cost < best) {
                 best = cost;
@@ -926,7 +941,13 @@ struct Engine final : EngineBase {
         const int maxblocks = per_sm * nsm;
         const int bpw = 32 / var().L;
         const int64_t groups = (N + bpw - 1) / bpw;
-        const int64_t want = std::max<int64_t>(1, (groups + blk / 32 - 1) / (blk / 32));
+        // groups that one block per SM holds are spread over every SM: a warp's
+        // chain is shorter the fewer warps share its SM (FP32, N = 1024: 8.4 us
+        // a step in 32 blocks of 8 warps, 8.0 in 128 of 2; FP64 9.7 and 8.3)
+        step_blk = blk;
+        if (groups <= (int64_t)nsm * (blk / 32))
+            step_blk = 32 * (int)std::max<int64_t>(1, (groups + nsm - 1) / nsm);
+        const int64_t want = std::max<int64_t>(1, (groups + step_blk / 32 - 1) / (step_blk / 32));
         step_grid = (int)std::min<int64_t>(want, maxblocks);
         return FCC_OK;
     }
@@ -1027,7 +1048,7 @@ struct Engine final : EngineBase {
         DevPtrs<T> d = ptrs();
         int p0 = par();
         void* args[] = {&d, &nsteps, &p0};
-        CUDA_TRY(cudaLaunchCooperativeKernel(step_kernel(), dim3(step_grid), dim3(var().blk), args, stage_bytes(), stream));
+        CUDA_TRY(cudaLaunchCooperativeKernel(step_kernel(), dim3(step_grid), dim3(step_blk), args, stage_bytes(), stream));
         gstep += nsteps;
         ++last_launches;
         return FCC_OK;
