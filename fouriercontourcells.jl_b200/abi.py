@@ -10,6 +10,7 @@ numpy arrays behind an ``fcc_bodies_host``.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import numpy as np
 
@@ -247,6 +248,15 @@ def direct_host(b: Bodies, writable: bool = False):
     return FccBodiesHost(n, c.shape[0], dptr(f["x"]), dptr(f["y"]), dptr(f["theta"]), iptr(f["imgx"]),
                          iptr(f["imgy"]), c.ctypes.data_as(c_double_p), dptr(f["R0"]), iptr(f["type"]),
                          iptr(f["parent"]))
+
+
+_BODIES_HOST = struct.Struct("@qi4x9P")
+
+
+def bodies_host_at(n: int, ncoef: int, *addresses) -> FccBodiesHost:
+    """An ``fcc_bodies_host`` over arrays at the given addresses (x, y, theta,
+    imgx, imgy, coef, R0, type, parent)."""
+    return FccBodiesHost.from_buffer_copy(_BODIES_HOST.pack(n, ncoef, *addresses))
 
 
 def bodies_over(block: np.ndarray, n: int, ncoef: int) -> Bodies:

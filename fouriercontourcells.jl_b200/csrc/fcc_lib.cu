@@ -1249,43 +1249,67 @@ struct Engine final : EngineBase {
         return sync_stream();
     }
 
+    // sim.grad: k_store_gradients widens and repacks on the device, into the
+    // caller's page-locked arrays in place, or (other memory) through one
+    // device area, an array at a time.
     fcc_status get_gradients(const fcc_gradients_host* o) override {
         if (!o) return fail(FCC_ERR_ARGUMENT, "null argument");
-        if (!P.p) FCC_TRY(ensure_diag());
+        if (N == 0) return FCC_OK;
+        FCC_TRY(ensure_diag());
         const size_t n = (size_t)N;
-        std::vector<T> a;
-        auto copy_nodes = [&](DBuf<T>& src, double* dst) -> fcc_status {
-            if (!dst) return FCC_OK;
-            FCC_TRY(fetch(src.p, n * nth, a));
-            FCC_TRY(sync_stream());
-            for (size_t q = 0; q < n * nth; ++q) dst[q] = (double)a[q];
+        GradOut<T> g{};
+        double* const node_out[4] = {o->GR, o->GD, o->GDD, o->P};
+        double* const body_out[4] = {o->gx, o->gy, o->gtheta, o->Ebody};
+        double* const coef_out[2] = {o->glab, o->gcoef};
+        const DBuf<T>* const node[4] = {&GR, &GD, &GDD, &P};
+        const DBuf<T>* const body[4] = {&gx, &gy, &gth, &E};
+        const DBuf<T>* const coefs[2] = {&glab, &gcoef};
+        for (int b = 0; b < 4; ++b) g.node[b] = node[b]->p, g.body[b] = body[b]->p;
+        for (int b = 0; b < 2; ++b) g.coef[b] = coefs[b]->p;
+        const int grid = (int)std::min<int64_t>((N * nth + 255) / 256, (int64_t)nsm * 8);
+        auto store = [&](const GradOut<T>& q) -> fcc_status {
+            k_store_gradients<T><<<grid, 256, 0, stream>>>(q, (long long)N, nth, nc, K);
+            CUDA_TRY(cudaGetLastError());
             return FCC_OK;
         };
-        auto copy_vec = [&](DBuf<T>& src, double* dst) -> fcc_status {
-            if (!dst) return FCC_OK;
-            FCC_TRY(fetch(src.p, n, a));
-            FCC_TRY(sync_stream());
-            for (size_t q = 0; q < n; ++q) dst[q] = (double)a[q];
+        GradOut<T> v = g;
+        bool in_place = true;
+        auto view = [&](double* host, double*& dev) {
+            dev = mapped_view(host);
+            in_place = in_place && (!host || dev);
+        };
+        for (int b = 0; b < 4; ++b) view(node_out[b], v.node_out[b]), view(body_out[b], v.body_out[b]);
+        for (int b = 0; b < 2; ++b) view(coef_out[b], v.coef_out[b]);
+        if (in_place) {
+            FCC_TRY(store(v));
+            return sync_stream();
+        }
+        DBuf<double> area;
+        FCC_TRY(area.alloc(n * (size_t)std::max(nth, nc), stream));
+        auto one = [&](const GradOut<T>& q, double* host, size_t count) -> fcc_status {
+            FCC_TRY(store(q));
+            CUDA_TRY(cudaMemcpyAsync(host, area.p, count * sizeof(double), cudaMemcpyDeviceToHost, stream));
             return FCC_OK;
         };
-        auto copy_coef = [&](DBuf<T>& src, double* dst) -> fcc_status {
-            if (!dst) return FCC_OK;
-            FCC_TRY(fetch(src.p, n * NCM, a));
-            FCC_TRY(sync_stream());
-            coef_out(a.data(), dst);
-            return FCC_OK;
-        };
-        FCC_TRY(copy_nodes(GR, o->GR));
-        FCC_TRY(copy_nodes(GD, o->GD));
-        FCC_TRY(copy_nodes(GDD, o->GDD));
-        FCC_TRY(copy_nodes(P, o->P));
-        FCC_TRY(copy_vec(gx, o->gx));
-        FCC_TRY(copy_vec(gy, o->gy));
-        FCC_TRY(copy_vec(gth, o->gtheta));
-        FCC_TRY(copy_coef(glab, o->glab));
-        FCC_TRY(copy_coef(gcoef, o->gcoef));
-        FCC_TRY(copy_vec(E, o->Ebody));
-        return FCC_OK;
+        for (int b = 0; b < 4; ++b) {
+            GradOut<T> q = g;
+            if (node_out[b]) {
+                q.node_out[b] = area.p;
+                FCC_TRY(one(q, node_out[b], n * nth));
+                q.node_out[b] = nullptr;
+            }
+            if (body_out[b]) {
+                q.body_out[b] = area.p;
+                FCC_TRY(one(q, body_out[b], n));
+            }
+        }
+        for (int b = 0; b < 2; ++b)
+            if (coef_out[b]) {
+                GradOut<T> q = g;
+                q.coef_out[b] = area.p;
+                FCC_TRY(one(q, coef_out[b], n * nc));
+            }
+        return sync_stream();
     }
 
     fcc_status get_geometry(const fcc_geometry_host* o) override {
@@ -1426,6 +1450,93 @@ struct Engine final : EngineBase {
 };
 
 // ------------------------------------------------- stateless entry points
+// Device arrays, stream and page-locked staging of one stateless neighbour
+// build, kept for the next one: twenty device allocations and their release
+// took 3 ms of a call whose kernels take 0.1.
+template <class T>
+struct ListWork {
+    struct Head {  // uploaded in one copy
+        SimDesc<T> desc;
+        GridSync sync;
+        long long clock, builds;
+        int flags, maxcount;
+    };
+    int device = 0;
+    cudaStream_t st = nullptr;
+    size_t n = 0, cells = 0, ids = 0;
+    DBuf<T> rec;
+    DBuf<int> sim_of, cellid, slot, perm, nb_count, nb_idx, cstart, cstop, ccount, cell_sim, out;
+    DBuf<double> in;
+    DBuf<Head> head;
+    Head* head_h = nullptr;
+    double* in_h = nullptr;
+    size_t in_cap = 0;
+    static constexpr size_t STAGED = 1 << 20;  // bodies whose inputs are staged in page-locked memory
+
+    ~ListWork() {
+        if (st) cudaStreamSynchronize(st);
+        if (head_h) cudaFreeHost(head_h);
+        if (in_h) cudaFreeHost(in_h);
+        if (st) cudaStreamDestroy(st);
+    }
+    fcc_status reserve(size_t n_, size_t cells_, size_t ids_) {
+        if (!st) {
+            CUDA_TRY(cudaGetDevice(&device));
+            CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+            CUDA_TRY(cudaMallocHost(&head_h, sizeof(Head)));
+            FCC_TRY(head.alloc(1, st));
+        }
+        if (n_ > n) {
+            FCC_TRY(rec.alloc(n_ * RECW, st));
+            for (DBuf<int>* b : {&sim_of, &cellid, &slot, &perm, &nb_count}) FCC_TRY(b->alloc(n_, st));
+            n = n_;
+        }
+        if (cells_ > cells) {  // ccount is zero between builds (phase_scan clears it)
+            for (DBuf<int>* b : {&cstart, &cstop, &ccount, &cell_sim}) FCC_TRY(b->alloc(cells_, st));
+            cells = cells_;
+        }
+        if (ids_ > ids) {
+            FCC_TRY(nb_idx.alloc(ids_, st));
+            ids = ids_;
+        }
+        return FCC_OK;
+    }
+    size_t bytes() const {
+        return n * (RECW * sizeof(T) + 5 * sizeof(int)) + cells * 4 * sizeof(int) + ids * sizeof(int) +
+               out.n * sizeof(int) + in.n * sizeof(double) + in_cap * sizeof(double);
+    }
+};
+
+// The workspaces not in use: at most KEEP of at most KEEP_BYTES each; every
+// call works on one of its own, so calls on several threads do not meet.
+template <class T>
+struct ListWorks {
+    static constexpr size_t KEEP = 2, KEEP_BYTES = (size_t)128 << 20;
+    std::mutex m;
+    std::vector<std::unique_ptr<ListWork<T>>> idle;
+    static ListWorks& all() {
+        static ListWorks* w = new ListWorks;  // never destroyed: the driver may be gone before static destructors
+        return *w;
+    }
+    std::unique_ptr<ListWork<T>> take() {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        std::lock_guard<std::mutex> lk(m);
+        for (size_t k = 0; k < idle.size(); ++k)
+            if (idle[k]->device == dev) {
+                auto w = std::move(idle[k]);
+                idle.erase(idle.begin() + (long)k);
+                return w;
+            }
+        return std::make_unique<ListWork<T>>();
+    }
+    void give(std::unique_ptr<ListWork<T>> w) {
+        if (w->bytes() > KEEP_BYTES) return;
+        std::lock_guard<std::mutex> lk(m);
+        if (idle.size() < KEEP) idle.push_back(std::move(w));
+    }
+};
+
 template <class T>
 fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const double* rmax, double Lx, double Ly,
                              double cutoff, double range, int32_t cap, int32_t* cellid_o, int32_t* perm_o,
@@ -1433,12 +1544,6 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
     if (n < 0 || cap < 1) return fail(FCC_ERR_ARGUMENT, "n must be >= 0 and cap >= 1");
     if (n == 0) return FCC_OK;
     if (n > (1 << 27)) return fail(FCC_ERR_UNSUPPORTED, "at most 2^27 bodies");
-    cudaStream_t st;
-    CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    struct StreamGuard {
-        cudaStream_t s;
-        ~StreamGuard() { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
-    } guard{st};
     SimDesc<T> s{};
     s.Lx = (T)Lx;
     s.Ly = (T)Ly;
@@ -1455,91 +1560,97 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
     s.nbrange = (T)range;
     s.skin = T(0);
     const size_t N = (size_t)n, C = (size_t)ncx * ncy;
-    DBuf<SimDesc<T>> sims;
-    DBuf<T> rec, xd, yd, rd;
-    DBuf<int> sim_of, cellid, slot, perm, cstart, cstop, ccount, cell_sim, nb_idx, nb_count, flags, maxcount;
-    DBuf<long long> clock, builds;
-    DBuf<GridSync> sync;
-    FCC_TRY(sims.upload(std::vector<SimDesc<T>>{s}, st));
-    std::vector<T> hx(N), hy(N), hr(N);
-    for (size_t i = 0; i < N; ++i) hx[i] = (T)x[i], hy[i] = (T)y[i], hr[i] = (T)rmax[i];
-    FCC_TRY(xd.upload(hx, st));
-    FCC_TRY(yd.upload(hy, st));
-    FCC_TRY(rd.upload(hr, st));
-    FCC_TRY(rec.alloc(N * RECW, st));
-    FCC_TRY(sim_of.alloc(N, st));
-    FCC_TRY(cellid.alloc(N, st));
-    FCC_TRY(slot.alloc(N, st));
-    FCC_TRY(perm.alloc(N, st));
-    FCC_TRY(cstart.alloc(C, st));
-    FCC_TRY(cstop.alloc(C, st));
-    FCC_TRY(ccount.alloc(C, st));
-    FCC_TRY(cell_sim.alloc(C, st));
-    FCC_TRY(nb_idx.alloc(N * cap, st));
-    FCC_TRY(nb_count.alloc(N, st));
-    FCC_TRY(flags.upload(std::vector<int>{F_ACTIVE | F_CONTACT | F_NEED}, st));
-    FCC_TRY(maxcount.alloc(1, st));
-    FCC_TRY(clock.alloc(1, st));
-    FCC_TRY(builds.alloc(1, st));
-    FCC_TRY(sync.upload(std::vector<GridSync>{GridSync{0, 0, 0, 1}}, st));
+    std::unique_ptr<ListWork<T>> w = ListWorks<T>::all().take();  // given back only after a call without errors
+    FCC_TRY(w->reserve(N, C, N * cap));
+    cudaStream_t st = w->st;
+    *w->head_h = {s, GridSync{0, 0, 0, 1}, 0, 0, F_ACTIVE | F_CONTACT | F_NEED, 0};
+    CUDA_TRY(cudaMemcpyAsync(w->head.p, w->head_h, sizeof(typename ListWork<T>::Head), cudaMemcpyHostToDevice, st));
+    // inputs: page-locked ones are read in place, others through page-locked
+    // staging (or, in large numbers, a device area)
+    const double *xd = mapped_view(x), *yd = mapped_view(y), *rd = mapped_view(rmax);
+    if (!(xd && yd && rd)) {
+        if (N <= ListWork<T>::STAGED) {
+            if (w->in_cap < 3 * N) {
+                if (w->in_h) cudaFreeHost(w->in_h);
+                w->in_h = nullptr;
+                w->in_cap = 0;
+                CUDA_TRY(cudaMallocHost(&w->in_h, 3 * N * sizeof(double)));
+                w->in_cap = 3 * N;
+            }
+            std::memcpy(w->in_h, x, N * sizeof(double));
+            std::memcpy(w->in_h + N, y, N * sizeof(double));
+            std::memcpy(w->in_h + 2 * N, rmax, N * sizeof(double));
+            xd = mapped_view(w->in_h);
+        } else {
+            if (w->in.n < 3 * N) FCC_TRY(w->in.alloc(3 * N, st));
+            CUDA_TRY(cudaMemcpyAsync(w->in.p, x, N * sizeof(double), cudaMemcpyHostToDevice, st));
+            CUDA_TRY(cudaMemcpyAsync(w->in.p + N, y, N * sizeof(double), cudaMemcpyHostToDevice, st));
+            CUDA_TRY(cudaMemcpyAsync(w->in.p + 2 * N, rmax, N * sizeof(double), cudaMemcpyHostToDevice, st));
+            xd = w->in.p;
+        }
+        if (!xd) return fail(FCC_ERR_CUDA, "page-locked staging is not mapped");
+        yd = xd + N;
+        rd = xd + 2 * N;
+    }
     DevPtrs<T> d{};
-    d.sims = sims.p;
+    d.sims = &w->head.p->desc;
     d.nsims = 1;
     d.Ntot = (int)N;
     d.Ctot = (int)C;
     d.cap = cap;
-    d.sim_of = sim_of.p;
-    d.rec0 = rec.p;
-    d.rec1 = rec.p;
-    d.cellid = cellid.p;
-    d.slot = slot.p;
-    d.perm = perm.p;
-    d.cstart = cstart.p;
-    d.cstop = cstop.p;
-    d.ccount = ccount.p;
-    d.cell_sim = cell_sim.p;
-    d.nb_idx = nb_idx.p;
-    d.nb_count = nb_count.p;
-    d.flags = flags.p;
-    d.maxcount = maxcount.p;
-    d.clock = clock.p;
-    d.builds = builds.p;
-    d.sync = sync.p;
+    d.sim_of = w->sim_of.p;
+    d.rec0 = w->rec.p;
+    d.rec1 = w->rec.p;
+    d.cellid = w->cellid.p;
+    d.slot = w->slot.p;
+    d.perm = w->perm.p;
+    d.cstart = w->cstart.p;
+    d.cstop = w->cstop.p;
+    d.ccount = w->ccount.p;
+    d.cell_sim = w->cell_sim.p;
+    d.nb_idx = w->nb_idx.p;
+    d.nb_count = w->nb_count.p;
+    d.flags = &w->head.p->flags;
+    d.maxcount = &w->head.p->maxcount;
+    d.clock = &w->head.p->clock;
+    d.builds = &w->head.p->builds;
+    d.sync = &w->head.p->sync;
     const int grid = (int)((N + 255) / 256);
-    k_pack_head<T><<<grid, 256, 0, st>>>(rec.p, xd.p, yd.p, rd.p, (int)N);
+    k_pack_head<T><<<grid, 256, 0, st>>>(d.rec0, xd, yd, rd, (int)N);
     k_phase_count<T><<<grid, 256, 0, st>>>(d, 0);
     k_phase_scan<T><<<1, 1024, 0, st>>>(d);
     k_phase_scatter<T><<<grid, 256, 0, st>>>(d);
     k_phase_sort<T><<<(int)((C + 255) / 256), 256, 0, st>>>(d);
     k_phase_neighbors<T><<<neighbor_grid(N), 256, 0, st>>>(d, 0);
     CUDA_TRY(cudaGetLastError());
-    std::vector<int> a, b, cnt;
-    a.resize(N);
-    CUDA_TRY(cudaMemcpyAsync(a.data(), cellid.p, N * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    for (size_t i = 0; i < N; ++i) cellid_o[i] = a[i] + 1;
-    CUDA_TRY(cudaMemcpyAsync(a.data(), perm.p, N * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    for (size_t i = 0; i < N; ++i) perm_o[i] = a[i] + 1;
-    a.resize(C);
-    b.resize(C);
-    CUDA_TRY(cudaMemcpyAsync(a.data(), cstart.p, C * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(b.data(), cstop.p, C * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    for (size_t c = 0; c < C; ++c) {
-        const bool empty = b[c] <= a[c];
-        start_o[c] = empty ? 1 : a[c] + 1;
-        stop_o[c] = empty ? 0 : b[c];
+    // results: written into page-locked arrays in place, others copied from a
+    // device area
+    int32_t* const host[6] = {cellid_o, perm_o, start_o, stop_o, idx_o, count_o};
+    const size_t len[6] = {N, N, C, C, N * cap, N};
+    int* dev[6];
+    bool in_place = true;
+    size_t total = 0;
+    for (int k = 0; k < 6; ++k) {
+        dev[k] = mapped_view(host[k]);
+        in_place = in_place && dev[k];
+        total += len[k];
     }
-    cnt.resize(N);
-    a.resize(N * cap);
-    CUDA_TRY(cudaMemcpyAsync(cnt.data(), nb_count.p, N * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(a.data(), nb_idx.p, N * cap * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    for (size_t i = 0; i < N; ++i) {
-        count_o[i] = cnt[i];
-        for (int q = 0; q < cap; ++q) idx_o[i * cap + q] = q < cnt[i] ? a[i * cap + q] + 1 : 0;
+    if (!in_place) {
+        if (w->out.n < total) FCC_TRY(w->out.alloc(total, st));
+        size_t off = 0;
+        for (int k = 0; k < 6; ++k) {
+            dev[k] = w->out.p + off;
+            off += len[k];
+        }
     }
+    const int sgrid = (int)std::min<size_t>((N * cap + 255) / 256, (size_t)148 * 8);
+    k_store_lists<T><<<sgrid, 256, 0, st>>>(d, ListOut{dev[0], dev[1], dev[2], dev[3], dev[4], dev[5]});
+    CUDA_TRY(cudaGetLastError());
+    if (!in_place)
+        for (int k = 0; k < 6; ++k)
+            CUDA_TRY(cudaMemcpyAsync(host[k], dev[k], len[k] * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    ListWorks<T>::all().give(std::move(w));
     return FCC_OK;
 }
 

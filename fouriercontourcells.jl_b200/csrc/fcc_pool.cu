@@ -1005,7 +1005,15 @@ struct Pool final : PoolBase {
             if (o->n != N || o->ncoef != P.nc) return fail(FCC_ERR_DIMENSION, "state buffers do not match the simulation");
             Arena<T>& a = *A;
             const size_t n = (size_t)N;
-            if (n > 0) {
+            double *vx = mapped_view(o->x), *vy = mapped_view(o->y), *vth = mapped_view(o->theta), *vc = mapped_view(o->coef);
+            int *vix = mapped_view(o->imgx), *viy = mapped_view(o->imgy);
+            const bool in_place = (!o->x || vx) && (!o->y || vy) && (!o->theta || vth) && (!o->coef || vc) &&
+                                  (!o->imgx || vix) && (!o->imgy || viy);
+            if (n > 0 && in_place) {  // page-locked arrays: written by the kernel, one launch and no copy
+                k_store_host<T><<<(int)std::min<size_t>((n * P.nc + 255) / 256, (size_t)nsm * 8), 256, 0, stream>>>(
+                    ptrs(), par(), (int)S.off, (int)n, vx, vy, vth, vc, P.nc, P.K, vix, viy);
+                CUDA_TRY(cudaGetLastError());
+            } else if (n > 0) {
                 FCC_TRY(st_xch.reserve(n * (3 + (size_t)P.nc), stream));
                 double* dx = st_xch.p();
                 k_store_host<T><<<(int)std::min<size_t>((n * P.nc + 255) / 256, (size_t)nsm * 8), 256, 0, stream>>>(

@@ -13,7 +13,7 @@ import math
 import numpy as np
 
 from . import abi
-from .simulation import native_library
+from .simulation import native_library, result_arrays
 
 
 def philox_noise(seed: int, draw: int, n: int, T=np.float64, lib=None, prefix="fcc_"):
@@ -57,9 +57,14 @@ def build_neighbors(x, y, rmax, Lx, Ly, cutoff, range_, cap=32, T=np.float64, li
     Lxt = float(np.float32(Lx)) if T32 else float(Lx)
     Lyt = float(np.float32(Ly)) if T32 else float(Ly)
     ncx, ncy = grid_dims(Lxt, Lyt, cutoff)
-    cellid, perm, count = (np.zeros(n, np.int32) for _ in range(3))
-    start, stop = np.zeros(ncx * ncy, np.int32), np.zeros(ncx * ncy, np.int32)
-    idx = np.zeros((n, cap), np.int32)
+    if n:
+        i = np.int32
+        cellid, perm, count, start, stop, idx = result_arrays(lib, *(((n,), i),) * 3, *(((ncx * ncy,), i),) * 2,
+                                                              ((n, cap), i))
+    else:  # the library writes nothing
+        cellid, perm, count = (np.zeros(0, np.int32) for _ in range(3))
+        start, stop = np.zeros(ncx * ncy, np.int32), np.zeros(ncx * ncy, np.int32)
+        idx = np.zeros((0, cap), np.int32)
     st = getattr(lib, prefix + "build_neighbors")(abi.precision_bits(T), n, abi.dptr(x), abi.dptr(y), abi.dptr(rmax),
                                                  float(Lx), float(Ly), float(cutoff), float(range_), int(cap),
                                                  abi.iptr(cellid), abi.iptr(perm), abi.iptr(start), abi.iptr(stop),

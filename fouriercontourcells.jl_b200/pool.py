@@ -19,7 +19,7 @@ import numpy as np
 
 from . import abi
 from .model import ArgumentError, Bodies, PoolFull
-from .simulation import native_library
+from .simulation import native_library, result_bodies
 
 _POOL_SIG = {
     "pool_bytes": [C.POINTER(abi.FccPoolParams), C.POINTER(C.c_int64)],
@@ -200,10 +200,9 @@ class Pool:
         if slot not in self._slots:
             raise ArgumentError(f"pool: no simulation in slot {slot}")
         n, ncoef, _, _ = self._slots[slot]
-        buf = abi.BodiesBuffer(n, ncoef)
+        b, host = result_bodies(self._lib, n, ncoef)
         clk, t, stp = C.c_int64(), C.c_double(), C.c_int64()
-        self._call("pool_get_state", self._h, int(slot), C.byref(buf.s), C.byref(clk), C.byref(t), C.byref(stp))
-        b = Bodies(buf.x, buf.y, buf.theta, buf.imgx, buf.imgy, buf.coefT.T, buf.R0, buf.type, buf.parent)
+        self._call("pool_get_state", self._h, int(slot), C.byref(host), C.byref(clk), C.byref(t), C.byref(stp))
         return b, clk.value, t.value, stp.value
 
     def bodies(self, slot: int) -> Bodies:

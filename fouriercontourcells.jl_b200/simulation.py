@@ -15,7 +15,9 @@ and fails loudly when that library is missing: there is no CPU fallback.
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
+import threading
 import weakref
 from collections import namedtuple
 
@@ -57,6 +59,91 @@ def native_library():
         lib.fcc_host_free.restype = C.c_int32
         _LIB = lib
     return _LIB
+
+
+class _ResultBlocks:
+    """Page-locked memory of the arrays that queries return (states, gradient
+    buffers, neighbour lists), which the device then writes in place: the
+    kernel that widens and repacks a result writes it across PCIe once, with
+    no staging copy and no host pass.  A block goes back when the last array
+    over it is collected and is handed out again for the next result of its
+    size.  At most ``LIMIT`` bytes are page-locked at a time, blocks in use
+    included (a program that keeps every snapshot gets ordinary arrays beyond
+    that: ``take`` returns None)."""
+
+    LIMIT = 256 << 20
+
+    def __init__(self):
+        self._lock = threading.RLock()  # a collection may give a block back inside take
+        self._idle = {}
+        self._total = 0
+
+    @staticmethod
+    def size_of(nbytes: int) -> int:
+        step = 1 << max(12, nbytes.bit_length() - 4)  # at most one eighth wasted
+        return -(-nbytes // step) * step
+
+    def take(self, lib, nbytes: int):
+        """A uint8 array of at least nbytes, or None."""
+        size = self.size_of(max(1, nbytes))
+        with self._lock:
+            idle = self._idle.get(size)
+            if idle:
+                ptr = idle.pop()
+            else:
+                while self._total + size > self.LIMIT and any(self._idle.values()):
+                    other = next(k for k, v in self._idle.items() if v)
+                    lib.fcc_host_free(self._idle[other].pop())
+                    self._total -= other
+                p = C.c_void_p()
+                if self._total + size > self.LIMIT or lib.fcc_host_alloc(size, C.byref(p)) != abi.FCC_OK:
+                    return None
+                ptr = p.value
+                self._total += size
+        block = np.frombuffer((C.c_uint8 * size).from_address(ptr), dtype=np.uint8)
+        weakref.finalize(block, self._give, ptr, size).atexit = False
+        return block
+
+    def _give(self, ptr, size):
+        with self._lock:
+            self._idle.setdefault(size, []).append(ptr)
+
+
+_BLOCKS = _ResultBlocks()
+
+
+def result_arrays(lib, *shapes):
+    """Arrays, one per (shape, dtype), for the library to fill: over one
+    page-locked block where there is room for it (their contents are then
+    whatever the block held), else zeros."""
+    sizes = [math.prod(shape) * dt().itemsize for shape, dt in shapes]
+    block = _BLOCKS.take(lib, sum(-(-n // 64) * 64 for n in sizes)) if hasattr(lib, "fcc_host_alloc") else None
+    if block is None:
+        return [np.zeros(shape, dt) for shape, dt in shapes]
+    out, off = [], 0
+    for (shape, dt), n in zip(shapes, sizes):
+        out.append(block[off:off + n].view(dt).reshape(shape))
+        off += -(-n // 64) * 64
+    return out
+
+
+def result_bodies(lib, n: int, ncoef: int):
+    """A ``Bodies`` for the library to fill (as ``result_arrays``) and the
+    ``fcc_bodies_host`` over it."""
+    d, k = -(-8 * n // 64) * 64, -(-4 * n // 64) * 64  # bytes of a vector of doubles, of ints
+    # x, y, θ, R0, the ints, then the coefficients
+    ends = [0, d, 2 * d, 3 * d, 4 * d, 4 * d + k, 4 * d + 2 * k, 4 * d + 3 * k, 4 * d + 4 * k]
+    block = _BLOCKS.take(lib, ends[8] + 8 * n * ncoef) if hasattr(lib, "fcc_host_alloc") else None
+    if block is None:
+        block = np.zeros(ends[8] + 8 * n * ncoef, np.uint8)
+    f, i, new = np.float64, np.int32, np.ndarray
+    x, y, θ, R0 = (new(n, f, block, o) for o in ends[:4])
+    imgx, imgy, typ, parent = (new(n, i, block, o) for o in ends[4:8])
+    coef = new((n, ncoef), f, block, ends[8]).T
+    a = block.__array_interface__["data"][0]
+    host = abi.bodies_host_at(n, ncoef, a, a + d, a + 2 * d, a + ends[4], a + ends[5], a + ends[8], a + 3 * d,
+                              a + ends[6], a + ends[7])
+    return Bodies(x, y, θ, imgx, imgy, coef, R0, typ, parent), host
 
 
 def pinned_bodies(n: int, ncoef: int) -> Bodies:
@@ -197,9 +284,9 @@ class NativeSimulation:
                                     "ABI's layout (contiguous vectors, coef in Fortran order): see pinned_bodies")
             self._call("get_state", self._h, C.byref(h), None, None, None)
             return out
-        buf = abi.BodiesBuffer(self.N, self.ncoef)
-        self._call("get_state", self._h, C.byref(buf.s), None, None, None)
-        return Bodies(buf.x, buf.y, buf.theta, buf.imgx, buf.imgy, buf.coefT.T, buf.R0, buf.type, buf.parent)
+        b, host = result_bodies(self._lib, self.N, self.ncoef)
+        self._call("get_state", self._h, C.byref(host), None, None, None)
+        return b
 
     @property
     def bodies(self) -> Bodies:
@@ -239,14 +326,11 @@ class NativeSimulation:
     @property
     def grad(self) -> Gradients:
         N, nθ, nc = self.N, self.nθ, self.ncoef
-        a = {f: np.zeros((N, nθ)) for f in ("GR", "GD", "GDD", "P")}
-        v = {f: np.zeros(N) for f in ("gx", "gy", "gtheta", "Ebody")}
-        m = {f: np.zeros((N, nc)) for f in ("glab", "gcoef")}
-        g = abi.FccGradientsHost(*(abi.dptr(x) for x in (a["GR"], a["GD"], a["GDD"], a["P"], v["gx"], v["gy"],
-                                                           v["gtheta"], m["glab"], m["gcoef"], v["Ebody"])))
+        f = np.float64
+        a = result_arrays(self._lib, *(((N, nθ), f),) * 4, *(((N,), f),) * 3, *(((N, nc), f),) * 2, ((N,), f))
+        g = abi.FccGradientsHost(*(abi.dptr(x) for x in a))
         self._call("get_gradients", self._h, C.byref(g))
-        return Gradients(a["GR"].T, a["GD"].T, a["GDD"].T, a["P"].T, v["gx"], v["gy"], v["gtheta"],
-                         m["glab"].T, m["gcoef"].T, v["Ebody"])
+        return Gradients(*(x.T for x in a))
 
     @property
     def geom(self) -> Geometry:

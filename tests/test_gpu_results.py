@@ -1,0 +1,104 @@
+"""Results written by the device into page-locked arrays (marked ``gpu``):
+the same values as through ordinary memory (the path of a caller's own arrays,
+and of results beyond the page-locked limit), and a stateless neighbour build
+that keeps its workspace between calls of other sizes, precisions and threads.
+Integers and doubles that are only copied or widened: the tolerance is
+equality."""
+
+from concurrent.futures import ThreadPoolExecutor
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import fcc, oracle
+
+pytestmark = pytest.mark.gpu
+
+abi, simulation = fcc.simulation.abi, fcc.simulation
+
+
+def sim(T, n=(7, 8), maxmode=6, nθ=24):
+    bodies, box = fcc.hexagonal_monolayer(*n, packing=0.98, maxmode=maxmode, rng=2)
+    bodies.coef[1:, :] = 0.03 * np.random.default_rng(5).standard_normal((bodies.ncoef - 1, bodies.n))
+    return bodies, box, dict(types=(fcc.BodyType(v0=0.06, Dr=0.01, μab=0.1),),
+                             energies=(fcc.Tension(0.01), fcc.Overlap(1.0)), nθ=nθ, T=T, seed=3)
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("maxmode,nθ", [(6, 24), (10, 40), (3, 64)])
+def test_results_in_place_equal_copied_ones(T, maxmode, nθ, monkeypatch):
+    bodies, box, kw = sim(T, maxmode=maxmode, nθ=nθ)
+    s = fcc.Simulation(bodies, box, **kw).refresh()
+    s.run(3)
+    s.refresh()
+    grad, state = s.grad, s.bodies
+    monkeypatch.setattr(simulation, "_BLOCKS", simulation._ResultBlocks())
+    monkeypatch.setattr(simulation._ResultBlocks, "LIMIT", 0)
+    for a, b in zip(grad, s.grad):
+        assert a.shape == b.shape and np.array_equal(a, b)
+    other = s.bodies
+    for f in ("x", "y", "θ", "imgx", "imgy", "coef", "R0", "type", "parent"):
+        a, b = getattr(state, f), getattr(other, f)
+        assert a.dtype == b.dtype and np.array_equal(a, b), f
+    # some buffers only, in the caller's own memory
+    gx, glab = np.zeros(s.N), np.zeros((s.N, s.ncoef))
+    g = abi.FccGradientsHost(None, None, None, None, abi.dptr(gx), None, None, abi.dptr(glab), None, None)
+    s._call("get_gradients", s._h, C.byref(g))
+    assert np.array_equal(gx, grad.gx) and np.array_equal(glab.T, grad.glab)
+
+
+def test_result_blocks_are_bounded_and_reused(monkeypatch):
+    monkeypatch.setattr(simulation, "_BLOCKS", simulation._ResultBlocks())
+    monkeypatch.setattr(simulation._ResultBlocks, "LIMIT", 1 << 20)
+    blocks, lib = simulation._BLOCKS, fcc.native_library()
+    kept = [blocks.take(lib, 200_000) for _ in range(8)]
+    assert sum(k is not None for k in kept) == (1 << 20) // blocks.size_of(200_000)
+    assert blocks.take(lib, 200_000) is None
+    address = kept[0].ctypes.data
+    view = kept[0][10:20]
+    kept[0] = None
+    assert blocks.take(lib, 200_000) is None      # a view keeps the block
+    del view
+    again = blocks.take(lib, 200_000)
+    assert again.ctypes.data == address
+    kept.clear()
+    del again                                     # every block is idle
+    big = blocks.take(lib, 900_000)               # idle blocks of other sizes make room
+    assert big is not None and blocks._total <= 1 << 20
+
+
+def neighbors(seed, n, T, cap=32):
+    rng = np.random.default_rng(seed)
+    L = np.sqrt(3.5 * n) + 4
+    x, y = rng.random(n) * L, rng.random(n) * L * 1.1
+    rmax = 0.9 + 0.3 * rng.random(n)
+    return (x, y, rmax, L, L * 1.1, 3.0, 0.3), dict(cap=cap, T=T)
+
+
+def same(a, b):
+    for u, v in zip(a[:4], b[:4]):
+        assert np.array_equal(u, v)
+    assert np.array_equal(a[5], b[5])
+    # the oracle orders and fills the first `cap` entries; the rest are zero here
+    cap = a[4].shape[0]
+    for i in range(a[4].shape[1]):
+        k = min(a[5][i], cap)
+        assert np.array_equal(a[4][:k, i], b[4][:k, i]) and not a[4][k:, i].any()
+
+
+def test_neighbor_workspace_over_sizes_precisions_and_threads():
+    jobs = [neighbors(k, n, T, cap) for k, (n, T, cap) in enumerate(
+        [(700, np.float64, 32), (5, np.float64, 3), (9000, np.float32, 20), (1, np.float32, 1), (700, np.float64, 2),
+         (9001, np.float64, 40), (300, np.float32, 33)])]
+    want = [oracle.build_neighbors(*a, **k) for a, k in jobs]
+    for _ in range(2):
+        for (a, k), w in zip(jobs, want):
+            same(fcc.build_neighbors(*a, **k), w)
+    with ThreadPoolExecutor(4) as ex:
+        for got, w in zip(ex.map(lambda j: fcc.build_neighbors(*j[0], **j[1]), jobs * 3), want * 3):
+            same(got, w)
+    with pytest.raises(fcc.ArgumentError):
+        fcc.build_neighbors(*jobs[0][0][:5], -1.0, 0.3)
+    same(fcc.build_neighbors(*jobs[0][0], **jobs[0][1]), want[0])
