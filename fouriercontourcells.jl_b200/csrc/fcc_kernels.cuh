@@ -663,6 +663,11 @@ __device__ void phase_neighbors(const DevPtrs<T>& d, int par, int tid, int nthr,
 // L2 in the loop).  At packing 0.95 with the 0.3 skin a body lists 6-9.
 constexpr int NBMAX = 12;
 
+// FP32: floats between staged neighbour records (112 bytes: the 16-byte reads
+// of a body's lanes at different neighbours fall into different banks; at 96
+// bytes every fourth neighbour shared its banks).
+constexpr int SRECW = RECW + 4;
+
 #ifndef FCC_DYN
 #define FCC_DYN 1  // 1: FP32, one simulation: warps take their block's warp groups dynamically
 #endif
@@ -722,14 +727,14 @@ template <class T, int L>
 __host__ __device__ constexpr size_t stage_bytes_per_warp() {
     // FP64: 4 own and 4 x NBMAX64 neighbour records, the nodes' offsets and pressures, the own coefficients
     if (sizeof(T) == 8) return (4 * (1 + NBMAX64) * SREC64 + 3 * 5 * 32 + 4 * SCF64) * sizeof(T);
-    return (size_t)(32 / L) * (1 + NBMAX) * RECW * sizeof(T) + desc_slot_bytes<T>() + walk_bytes_per_warp<T, L>();
+    return (size_t)(32 / L) * (RECW + NBMAX * SRECW) * sizeof(T) + desc_slot_bytes<T>() + walk_bytes_per_warp<T, L>();
 }
 
 // the walk slots' place in a warp's stage (draw_ahead)
 template <class T, int L>
 __host__ __device__ constexpr int draw_ahead_slot() {
     return sizeof(T) == 8 ? 4 * (1 + NBMAX64) * SREC64
-                          : (32 / L) * (1 + NBMAX) * RECW + (int)(desc_slot_bytes<T>() / sizeof(T));
+                          : (32 / L) * (RECW + NBMAX * SRECW) + (int)(desc_slot_bytes<T>() / sizeof(T));
 }
 
 // ------------------------------------------------ tensor-core contractions
@@ -1424,7 +1429,7 @@ __device__ __forceinline__ void contact_lat(const T* snb, int n, int q0, int q1,
 #pragma unroll 2
         for (int qq = q0; qq < qe; ++qq) {
             T ox, oy, lim2, cA;
-            lds_head(snb + qq * RECW, ox, oy, lim2, cA);
+            lds_head(snb + qq * SRECW, ox, oy, lim2, cA);
             unsigned m = 0;
 #pragma unroll
             for (int sl = 0; sl < S; ++sl) {
@@ -1452,7 +1457,7 @@ __device__ __forceinline__ void contact_lat(const T* snb, int n, int q0, int q1,
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             sl[i] = bit[i] - (bit[i] / S) * S;
-            r[i] = snb + (q0 + bit[i] / S) * RECW;
+            r[i] = snb + (q0 + bit[i] / S) * SRECW;
             T ox, oy, lim2;
             lds_head(r[i], ox, oy, lim2, cA[i]);
             const auto e = lds4(wsl + sl[i] * 4);
@@ -1509,6 +1514,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     constexpr bool MMA = ONE && sizeof(T) == 4 && L == 8 && S == 5 && !USER;
     constexpr bool MMA_S = MMA && FCC_MMA_SYNTH;
     constexpr int MPL = UpdatePre<T, L>::MPL;
+    constexpr int SRW = SRECW;
     const int lane = threadIdx.x & 31;
     const int l = lane & (L - 1);
     const int g = wg * BPW + lane / L;
@@ -1521,7 +1527,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         s = gf < d.Ntot ? __ldg(d.sim_of + gf) : -1;
         if (s < 0) return;
         if (s != cached) {  // the warp moved to another simulation: copy its descriptor
-            SimDesc<T>* wd = reinterpret_cast<SimDesc<T>*>(stage + (size_t)BPW * (1 + NBMAX) * RECW);
+            SimDesc<T>* wd = reinterpret_cast<SimDesc<T>*>(stage + (size_t)BPW * (RECW + NBMAX * SRW));
             const unsigned* src = reinterpret_cast<const unsigned*>(d.sims + s);
             unsigned* dst = reinterpret_cast<unsigned*>(wd);
             __syncwarp();
@@ -1531,7 +1537,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         }
     }
     const SimDesc<T>& P =
-        sim0 ? *sim0 : *reinterpret_cast<const SimDesc<T>*>(stage + (size_t)BPW * (1 + NBMAX) * RECW);
+        sim0 ? *sim0 : *reinterpret_cast<const SimDesc<T>*>(stage + (size_t)BPW * (RECW + NBMAX * SRW));
     const bool valid = sim0 ? g < d.Ntot : g < P.body_off + P.n;
     const int gg = valid ? g : (sim0 ? 0 : wg * BPW);
     const T* rc = rec_cur(d, par);
@@ -1539,7 +1545,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     // registers, the whole record to shared memory), neighbour count and ids,
     // simulation state, update operands
     T* own = stage + (size_t)(lane / L) * RECW;
-    T* snb = stage + (size_t)BPW * RECW + (size_t)(lane / L) * NBMAX * RECW;
+    T* snb = stage + (size_t)BPW * RECW + (size_t)(lane / L) * NBMAX * SRW;
     const T* grec = rc + (size_t)gg * RECW;
     T xi, yi, rmi, wf, a0r, th, r0;
     int cnt_raw;
@@ -1611,60 +1617,54 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     auto stage_batch = [&](int base, bool have) {  // have: ids holds the batch's ids
         const int npre = min(cnt - base, NBMAX);
         __syncwarp();  // every lane is done with the previous contents
-        if constexpr (LAT) {  // a record by the lanes of its body
+        // a record by the lanes of its body: whole lines (a record per lane took
+        // 32 lines an instruction; N = 16384 23.0 against 22.6 us a step)
 #pragma unroll
-            for (int u = 0; u < IDS; ++u)
-                if (!have && l + u * L < npre) ids[u] = ldcg(d.nb_idx + (size_t)gg * d.cap + base + l + u * L);
-            int j[NBMAX];
+        for (int u = 0; u < IDS; ++u)
+            if (!have && l + u * L < npre) ids[u] = ldcg(d.nb_idx + (size_t)gg * d.cap + base + l + u * L);
+        int j[NBMAX];
 #pragma unroll
-            for (int q = 0; q < NBMAX; ++q) j[q] = __shfl_sync(FULL, ids[q / L], q % L, L);
+        for (int q = 0; q < NBMAX; ++q) j[q] = __shfl_sync(FULL, ids[q / L], q % L, L);
 #pragma unroll
-            for (int q = 0; q < NBMAX; ++q)
-                if (q < npre && l < CH16)
-                    cp_async16(snb + q * RECW + l * (16 / sizeof(T)), rc + (size_t)j[q] * RECW + l * (16 / sizeof(T)));
-            cp_async_commit();
-            return;
-        }
+        for (int q = 0; q < NBMAX; ++q)
+            if (q < npre) {
+#pragma unroll
+                for (int c = 0; c < CH16; c += L)
+                    if (c + l < CH16)
+                        cp_async16(snb + q * SRW + (c + l) * (16 / sizeof(T)),
+                                   rc + (size_t)j[q] * RECW + (c + l) * (16 / sizeof(T)));
+            }
+        cp_async_commit();
+    };
+
+    const int wv = unpack_w(wf);
+    const int ti = wv & 7;
+    const int pi = wv >> 3;
+    // a batch once it has arrived: lane q replaces the head of record q by the
+    // minimum-image centre offset r_i - r_j, the squared reach and (without
+    // user terms) the pair's coupling, which the contact phases then read
+    // (worked out by every lane at every test and hit before: N = 16384 22.6
+    // against 22.2 us a step)
+    auto finish_batch = [&](int base) {
+        cp_async_wait_all();
+        __syncwarp();
+        const int npre = min(cnt - base, NBMAX);
 #pragma unroll
         for (int u = 0; u < IDS; ++u) {
             const int q = l + u * L;
             if (q < npre) {
-                const int j = base == 0 ? ids[u] : ldcg(d.nb_idx + (size_t)gg * d.cap + base + q);
-                const T* src = rc + (size_t)j * RECW;
-#pragma unroll
-                for (int c = 0; c < CH16; ++c) cp_async16(snb + q * RECW + c * (16 / sizeof(T)), src + c * (16 / sizeof(T)));
+                T* r = snb + q * SRW;
+                T xj, yj, rmj, wj;
+                lds_head(r, xj, yj, rmj, wj);
+                const int wjv = unpack_w(wj);
+                const T lim = rmj + P.crange;
+                r[R_X] = minimum_image_fast(xi - xj, P.Lx, P.invLx);
+                r[R_Y] = minimum_image_fast(yi - yj, P.Ly, P.invLy);
+                r[R_RMAX] = lim * lim;
+                if constexpr (!USER) r[R_W] = P.cA[(wjv >> 3) == pi ? 1 : 0][ti][wjv & 7];
             }
         }
-        cp_async_commit();
-    };
-    const int wv = unpack_w(wf);
-    const int ti = wv & 7;
-    const int pi = wv >> 3;
-    // LAT: a batch once it has arrived: lane q replaces the head of record q by
-    // the minimum-image centre offset r_i - r_j, the squared reach and the
-    // pair's coupling, which the contact phases then read
-    auto finish_batch = [&](int base) {
-        cp_async_wait_all();
         __syncwarp();
-        if constexpr (LAT) {
-            const int npre = min(cnt - base, NBMAX);
-#pragma unroll
-            for (int u = 0; u < IDS; ++u) {
-                const int q = l + u * L;
-                if (q < npre) {
-                    T* r = snb + q * RECW;
-                    T xj, yj, rmj, wj;
-                    lds_head(r, xj, yj, rmj, wj);
-                    const int wjv = unpack_w(wj);
-                    const T lim = rmj + P.crange;
-                    r[R_X] = minimum_image_fast(xi - xj, P.Lx, P.invLx);
-                    r[R_Y] = minimum_image_fast(yi - yj, P.Ly, P.invLy);
-                    r[R_RMAX] = lim * lim;
-                    r[R_W] = P.cA[(wjv >> 3) == pi ? 1 : 0][ti][wjv & 7];
-                }
-            }
-            __syncwarp();
-        }
     };
     stage_batch(0, true);
     int staged_base = 0;
@@ -1676,7 +1676,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     const int nch = ONE ? 1 : (nth + L * S - 1) / (L * S);
 
     // the warp's walk slots: also the transposition buffer of the tensor-core contractions
-    T* wbase = stage + (size_t)BPW * (1 + NBMAX) * RECW + desc_slot_bytes<T>() / sizeof(T);
+    T* wbase = stage + (size_t)BPW * (RECW + NBMAX * SRW) + desc_slot_bytes<T>() / sizeof(T);
     const float* mtab = MMA ? reinterpret_cast<const float*>(tab) + BASIS_NODES * KM * 4 : nullptr;
 
     // own lab coefficients are read from the staged record (modes outer,
@@ -1813,7 +1813,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     }
 
     finish_batch(0);
-    const T Lx = P.Lx, Ly = P.Ly, iLx = P.invLx, iLy = P.invLy, crange = P.crange;
+    const T Lx = P.Lx, Ly = P.Ly, iLx = P.invLx, iLy = P.invLy;
     const bool rewrap = P.rewrap != 0;
 
     T GRs[S], GDs[S];  // node gradients of the tensor-core pullback (0 beyond the contour; one chunk)
@@ -1823,7 +1823,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
 #pragma unroll
         for (int sl = 0; sl < S; ++sl) p[sl] = T(0);
         // per lane and node slot (R, cos, sin, pressure) for the hit walk
-        T* wsl = stage + (size_t)BPW * (1 + NBMAX) * RECW + desc_slot_bytes<T>() / sizeof(T) + (size_t)lane * S * 4;
+        T* wsl = stage + (size_t)BPW * (RECW + NBMAX * SRW) + desc_slot_bytes<T>() / sizeof(T) + (size_t)lane * S * 4;
         if (FCC_WALK_SMEM && S <= slots_of(L) && maxc > 0) {
 #pragma unroll
             for (int sl = 0; sl < S; ++sl) {
@@ -1853,27 +1853,29 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
                         contact_lat<T, S>(snb, cnt - base, q0, q1, R, C1, S1, vmask, rewrap, Lx, Ly, iLx, iLy, P.cB[ti], wsl);
                         continue;
                     }
-                    for (int qq = q0; qq < q1; ++qq) {
-                        if (base + qq < cnt) {
-                            T xj, yj, rmj, wj;
-                            lds_head(snb + qq * RECW, xj, yj, rmj, wj);
-                            const T dxc = minimum_image_fast(xi - xj, Lx, iLx);
-                            const T dyc = minimum_image_fast(yi - yj, Ly, iLy);
-                            const T lim = rmj + crange;
-                            const T lim2 = lim * lim;
-                            unsigned m = 0;  // this neighbour's hits over the lane's node slots
+                    auto test = [&](auto wrap) {
+                        for (int qq = q0; qq < q1; ++qq) {
+                            if (base + qq < cnt) {
+                                T dxc, dyc, lim2, wj;
+                                lds_head(snb + qq * SRW, dxc, dyc, lim2, wj);
+                                unsigned m = 0;  // this neighbour's hits over the lane's node slots
 #pragma unroll
-                            for (int sl = 0; sl < S; ++sl) {
-                                T dx = R[sl] * C1[sl] + dxc, dy = R[sl] * S1[sl] + dyc;
-                                if (rewrap) {
-                                    dx = minimum_image_fast(dx, Lx, iLx);
-                                    dy = minimum_image_fast(dy, Ly, iLy);
+                                for (int sl = 0; sl < S; ++sl) {
+                                    T dx = R[sl] * C1[sl] + dxc, dy = R[sl] * S1[sl] + dyc;
+                                    if (USER ? rewrap : decltype(wrap)::value) {
+                                        dx = minimum_image_fast(dx, Lx, iLx);
+                                        dy = minimum_image_fast(dy, Ly, iLy);
+                                    }
+                                    m |= (dx * dx + dy * dy <= lim2) ? (1u << sl) : 0u;
                                 }
-                                m |= (dx * dx + dy * dy <= lim2) ? (1u << sl) : 0u;
+                                hm |= (unsigned long long)(m & vmask) << ((qq - q0) * S);
                             }
-                            hm |= (unsigned long long)(m & vmask) << ((qq - q0) * S);
                         }
-                    }
+                    };
+                    // one loop for boxes that re-image every node, one without (a pool
+                    // of 64: 51.7 against 50.4 us a step); a single one with user terms
+                    if (!USER && rewrap) test(Flag<true>{});
+                    else test(Flag<false>{});
                     // (2) every lane walks its own hits in (neighbour, node) order, so
                     // each node sums its neighbours' g(d) in list order
                     // (src/energies/contact.jl:309-322)
@@ -1881,13 +1883,12 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
                     auto hit_value = [&](int bit, int& sl) -> T {
                         const int qq = q0 + bit / S;
                         sl = bit - (bit / S) * S;
-                        const T* nrec = snb + qq * RECW;
-                        T xj, yj, rmj, wj;
-                        lds_head(nrec, xj, yj, rmj, wj);
-                        const T dxc = minimum_image_fast(xi - xj, Lx, iLx);
-                        const T dyc = minimum_image_fast(yi - yj, Ly, iLy);
-                        const int wjv = unpack_w(wj);
-                        const T cAj = P.cA[(wjv >> 3) == pi ? 1 : 0][ti][wjv & 7];
+                        const T* nrec = snb + qq * SRW;
+                        T dxc, dyc, lim2, wj;
+                        lds_head(nrec, dxc, dyc, lim2, wj);
+                        T cAj;
+                        if constexpr (!USER) cAj = wj;
+                        else cAj = P.cA[(unpack_w(wj) >> 3) == pi ? 1 : 0][ti][unpack_w(wj) & 7];
                         T rr, rcs, rsn;
                         if constexpr (WS) {
                             const auto e = lds4(wsl + sl * 4);
@@ -1920,7 +1921,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
 #pragma unroll
                             for (int u = 0; u < MUT; ++u)
                                 if (u < P.nuc && ((P.uc_mask[u] >> ti) & 1u))
-                                    gv += fcc_user::contact_g<T>(P.uc_id[u], dd, ti + 1, (wjv & 7) + 1, (wjv >> 3) == pi,
+                                    gv += fcc_user::contact_g<T>(P.uc_id[u], dd, ti + 1, (unpack_w(wj) & 7) + 1, (unpack_w(wj) >> 3) == pi,
                                                                 P.uc_a[u], P.uc_b[u]);
                         }
                         return gv;
