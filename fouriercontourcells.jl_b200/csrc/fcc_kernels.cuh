@@ -671,9 +671,6 @@ constexpr int SRECW = RECW + 4;
 #ifndef FCC_DYN
 #define FCC_DYN 1  // 1: FP32, one simulation: warps take their block's warp groups dynamically
 #endif
-#ifndef FCC_FLAT_BARRIER
-#define FCC_FLAT_BARRIER 1  // 1: a lone simulation's step barrier polls its arrival counter (flat_barrier)
-#endif
 
 // FP32 single-chunk kernels read cos(n phi_k), sin(n phi_k) (and n times
 // them) of their contour nodes from a shared-memory table instead of running
@@ -2302,9 +2299,8 @@ __device__ __forceinline__ void lone_book_writes(const DevPtrs<T>& d, const Barr
 template <class T>
 __device__ __forceinline__ bool rebuild_prologue(const DevPtrs<T>& d, int par, int tid, int nthr, BarrierLocal& bl,
                                                  const SimDesc<T>* sim0, int* wl_area, int wl_cap) {
-    // the phases set F_VALID / F_FROZEN: a lone simulation's flags are re-read
-    auto keep = [&](unsigned) { return lone_sim(d) ? (bl.any | ((ldcg(d.flags) & 0xff) << 1)) : -1; };
-    if (FCC_FLAT_BARRIER && lone_sim(d)) {
+    auto keep = [](unsigned) { return -1; };
+    if (lone_sim(d)) {
         // a lone simulation: flat barriers, and each block tracks the flags the
         // phases set (F_VALID from the scan, F_FROZEN from an overflowing list,
         // voted at the last barrier) instead of re-reading them
@@ -2332,7 +2328,7 @@ __device__ __forceinline__ bool rebuild_prologue(const DevPtrs<T>& d, int par, i
     wl.m = -1;
     if (!sim0) wl = build_worklist(d, wl_area, wl_cap);
     const WorkList* wlp = wl.m >= 0 ? &wl : nullptr;
-    phase_count(d, par, tid, nthr, wlp, lone_sim(d) ? bl.any : -1);
+    phase_count(d, par, tid, nthr, wlp);
     if (!grid_barrier(d.sync, bl, keep)) return false;
     phase_scan(d, wlp);
     if (!grid_barrier(d.sync, bl, keep)) return false;
@@ -2406,7 +2402,8 @@ __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
 // within the block the warps take them statically, or (FP32, one simulation)
 // each warp its first and then the block's next untaken one.
 template <class T, int L, int S, bool ONE, bool SPLIT, int BLK, int MINB, bool USER = false>
-__global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, int par0) {
+__global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, int par0, LaunchStatus* status,
+                                                    long long ticket) {
     constexpr bool LAT = MINB == 1 && ONE && !SPLIT && L == 8 && S == 5;
     const int WPB = blockDim.x >> 5;  // at most BLK / 32
     const int warp = threadIdx.x >> 5;
@@ -2433,7 +2430,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
     __syncthreads();
     // a lone simulation's warps draw the normals of their first group of the
     // next step while they wait at the step barrier
-    const bool ahead = FCC_FLAT_BARRIER && !SPLIT && !USER && lone && sim0->has_noise;
+    const bool ahead = !SPLIT && !USER && lone && sim0->has_noise;
     bool drawn = false;
     // One block of registers per SM (MINB = 1): the kernels for grids that hold
     // at most one warp group per warp, where a group's chain of latencies is
@@ -2487,7 +2484,7 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
         // a lone simulation that stepped ticks its block-local clock inside the
         // barrier: the next step's warps read it for their noise
         const int tick = (lone && (f0 & F_ACTIVE) && !(f0 & (F_FROZEN | F_HOLD))) ? 1 : 0;
-        if (FCC_FLAT_BARRIER && lone) {
+        if (lone) {
             // every block decides the next step from the same counter value;
             // block 0 writes the global flags and clock
             // (the block barrier above is the flat barrier's entry barrier)
@@ -2508,15 +2505,17 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
             drawn = ahead;
             continue;
         }
-        if (!grid_barrier(
-                d.sync, bl, [&](unsigned rbs) { return bookkeeping(d, bl, rbs, sim0); }, rb,
-                [&](int code) {
-                    if (lone) lone_book_writes(d, bl, code);
-                },
-                tick))
-            return;
+        if (!grid_barrier(d.sync, bl, [&](unsigned rbs) { return bookkeeping(d, bl, rbs, sim0); }, rb)) return;
     }
-    if (FCC_FLAT_BARRIER && lone && threadIdx.x == 0) flat_end(d.sync);
+    if (lone && threadIdx.x == 0 && flat_end(d.sync) && status) {
+        // block 0's writes of the last step may still be under way: the clock
+        // from this block; the flags of the last barrier, plus what is set at any time
+        __threadfence();
+        status->flags = bl.flags | (ldcg(d.flags) & F_NONFINITE);
+        status->error = ld_acquire(&d.sync->error);
+        status->clock = bl.clock;
+        status->ticket = ticket;
+    }
 }
 
 // Self-test of the bounded barrier waits: the last block leaves without

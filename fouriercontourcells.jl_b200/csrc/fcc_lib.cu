@@ -669,6 +669,9 @@ struct Engine final : EngineBase {
     int ccap = 1, bcap = 1;
     Status* st_h = nullptr;  // pinned read-back of the run state
     Status* up_h = nullptr;  // pinned head written by load_state
+    LaunchStatus* ls_h = nullptr;  // pinned, written by the step kernel at the end of a launch
+    LaunchStatus* ls_d = nullptr;  // the device's address of it
+    long long ticket = 0;
     // state exchange with the host (set_state / get_state): the caller's
     // double arrays are copied as they are into one device area (x, y, theta,
     // coefficients in the reference's layout), and converted and repacked on
@@ -681,6 +684,7 @@ struct Engine final : EngineBase {
         if (stream) cudaStreamSynchronize(stream);
         if (st_h) cudaFreeHost(st_h);
         if (up_h) cudaFreeHost(up_h);
+        if (ls_h) cudaFreeHost(ls_h);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
@@ -755,6 +759,10 @@ struct Engine final : EngineBase {
         CUDA_TRY(cudaEventCreate(&ev1));
         CUDA_TRY(cudaMallocHost(&st_h, sizeof(Status)));
         CUDA_TRY(cudaMallocHost(&up_h, sizeof(Status)));
+        CUDA_TRY(cudaMallocHost(&ls_h, sizeof(LaunchStatus)));
+        *ls_h = LaunchStatus{};
+        ls_d = mapped_view(ls_h);
+        if (!ls_d) return fail(FCC_ERR_UNSUPPORTED, "page-locked memory is not mapped");
 
         N = sp.N;
         K = sp.K;
@@ -1047,7 +1055,8 @@ struct Engine final : EngineBase {
     fcc_status launch_steps(int nsteps) {
         DevPtrs<T> d = ptrs();
         int p0 = par();
-        void* args[] = {&d, &nsteps, &p0};
+        ++ticket;
+        void* args[] = {&d, &nsteps, &p0, &ls_d, &ticket};
         CUDA_TRY(cudaLaunchCooperativeKernel(step_kernel(), dim3(step_grid), dim3(step_blk), args, stage_bytes(), stream));
         gstep += nsteps;
         ++last_launches;
@@ -1068,12 +1077,22 @@ struct Engine final : EngineBase {
                 FCC_TRY(launch_steps(k));
                 remaining -= k;
             }
-            FCC_TRY(read_status());
-            account(st_h->clock);
-            const int64_t executed = st_h->clock - start;
+            // the kernel itself leaves its status for the host: no copy, one synchronisation
+            CUDA_TRY(cudaEventRecord(ev1, stream));
+            FCC_TRY(sync_stream());
+            LaunchStatus ls;
+            std::memcpy(&ls, ls_h, sizeof(ls));  // written by the device before the stream was done
+            if (ls.ticket != ticket || ls.error)
+                return fail(FCC_ERR_DEVICE, "a grid barrier wait timed out in the step kernel");
+            account(ls.clock);
+            const int64_t executed = ls.clock - start;
             done += executed;
-            if (st_h->flags & F_FROZEN) FCC_TRY(regrow());
-            else if (executed < requested) return fail(FCC_ERR_DEVICE, "step kernel did not advance the clock");
+            if (ls.flags & F_FROZEN) {
+                FCC_TRY(read_status());
+                FCC_TRY(regrow());
+            } else if (executed < requested) {
+                return fail(FCC_ERR_DEVICE, "step kernel did not advance the clock");
+            }
         }
         return FCC_OK;
     }
@@ -1093,8 +1112,6 @@ struct Engine final : EngineBase {
         const long long c0 = clock_h;
         CUDA_TRY(cudaEventRecord(ev0, stream));
         FCC_TRY(advance(n, eager ? 1 : 512));
-        CUDA_TRY(cudaEventRecord(ev1, stream));
-        CUDA_TRY(cudaEventSynchronize(ev1));
         float ms = 0;
         CUDA_TRY(cudaEventElapsedTime(&ms, ev0, ev1));
         last_ms = ms;

@@ -271,9 +271,9 @@ struct Pool final : PoolBase {
     std::vector<long long> graph_key;
     int64_t graph_launches = 0;
     // launch configuration
-    int variant = -1;  // -1: default (variant 0)
+    int variant = -1;  // -1: chosen by size (variant_index)
     int spl = 512;
-    int grid = 0;
+    int grid = 0, blk = 0;
     double last_ms = 0;
     int64_t last_launches = 0, last_body_steps = 0;
 
@@ -289,7 +289,20 @@ struct Pool final : PoolBase {
     }
 
     int par() const { return (int)(gstep & 1); }
-    const Variant& var() const { return VARIANTS[variant < 0 ? 0 : variant]; }
+    // Without a configured or tuned variant, the launch shape a lone simulation
+    // of this size would take among those of two blocks per SM (same bits), and
+    // in FP64 the one-round shape: us a step, 256- / 224-thread blocks, FP32 5240
+    // bodies in 24 members 22.7 / 20.7, 27 496 in 64 52.0 / 57.6, 37 904 in 40
+    // 65.5 / 63.8; FP64 5240 30.3 / 25.8, 27 496 69.4 / 69.4, 37 904 91.1 / 83.3.
+    int variant_index() const {
+        if (variant >= 0) return variant;
+        const int64_t groups = (Ntot + 3) / 4;
+        if (sizeof(T) == 8) return groups <= (int64_t)nsm * 8 ? 0 : 5;
+        if (nth > 40 || split()) return 0;
+        auto rounds = [&](int64_t warps) { return (double)((groups + warps - 1) / warps); };
+        return 0.97 * rounds((int64_t)nsm * 14) < rounds((int64_t)nsm * 16) ? 5 : 0;
+    }
+    const Variant& var() const { return VARIANTS[variant_index()]; }
     bool split() const { return nsplit > 0; }
     void* step_kernel() const { return (sizeof(T) == 4 ? var().f32 : var().f64)(nth <= var().L * var().S, split()); }
     size_t stage_bytes() const {
@@ -610,7 +623,9 @@ struct Pool final : PoolBase {
         if (per_sm < 1) return fail(FCC_ERR_UNSUPPORTED, "step kernel does not fit on an SM");
         const int bpw = 32 / var().L;
         const int64_t groups = (Ntot + bpw - 1) / bpw;
-        const int64_t want = std::max<int64_t>(1, (groups + var().blk / 32 - 1) / (var().blk / 32));
+        blk = var().blk;  // a grid that one block per SM holds is spread over every SM, as a lone simulation's
+        if (groups <= (int64_t)nsm * (blk / 32)) blk = 32 * (int)std::max<int64_t>(1, (groups + nsm - 1) / nsm);
+        const int64_t want = std::max<int64_t>(1, (groups + blk / 32 - 1) / (blk / 32));
         grid = (int)std::min<int64_t>(want, (int64_t)per_sm * nsm);
         return FCC_OK;
     }
@@ -689,8 +704,10 @@ struct Pool final : PoolBase {
         for (int64_t left = most; left > 0;) {
             int k = (int)std::min<int64_t>(spl, left);
             int p0 = (int)(g & 1);
-            void* args[] = {&d, &k, &p0};
-            CUDA_TRY(cudaLaunchCooperativeKernel(step_kernel(), dim3(grid), dim3(var().blk), args, stage_bytes(), stream));
+            LaunchStatus* no_status = nullptr;
+            long long no_ticket = 0;
+            void* args[] = {&d, &k, &p0, &no_status, &no_ticket};
+            CUDA_TRY(cudaLaunchCooperativeKernel(step_kernel(), dim3(grid), dim3(blk), args, stage_bytes(), stream));
             g += k;
             left -= k;
         }
@@ -703,7 +720,7 @@ struct Pool final : PoolBase {
         const int64_t nl = (most + spl - 1) / spl;
         if (use_graph && graph_ok) {
             const std::vector<long long> key = {(long long)(uintptr_t)A.get(), (long long)Ntot, (long long)Ctot,
-                                                (long long)grid, (long long)variant, (long long)split(),
+                                                (long long)grid, (long long)variant_index(), (long long)split(),
                                                 (long long)cap, (long long)par(), (long long)most, (long long)spl};
             if (key != graph_key) {
                 drop_graph();
@@ -903,7 +920,7 @@ struct Pool final : PoolBase {
         const std::vector<Slot> mirror = slots;
         const long long gstep0 = gstep;
         const int cap0 = cap, variant0 = variant;
-        const Variant& cur = VARIANTS[variant < 0 ? 0 : variant];
+        const Variant& cur = var();
         auto restore = [&]() -> fcc_status {
             if (A->cap != cap0) {
                 FCC_TRY(A->alloc((size_t)max_bodies, (size_t)max_cells, cap0, ccap, bcap, stream));
@@ -1091,7 +1108,7 @@ struct Pool final : PoolBase {
     }
 
     fcc_status variant_info(int32_t* v, int32_t* L, int32_t* S_, int32_t* blk, int32_t* minb, int32_t* g) override {
-        if (v) *v = variant < 0 ? 0 : variant;
+        if (v) *v = variant_index();
         if (L) *L = var().L;
         if (S_) *S_ = var().S;
         if (blk) *blk = var().blk;
