@@ -231,6 +231,8 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int IDS = (NBMAX64 + L - 1) / L;
     constexpr int MPL = 2;  // modes per lane
+    // slot of a staged neighbour's coupling: its record word, which user terms need, or its theta
+    constexpr int COUPLING = USER ? R_TH : R_W;
     const int lane = threadIdx.x & 31;
     const int l = lane & 7, tq = lane & 3, b = lane >> 3;
     const bool h = lane & 4;  // this lane's MMA row is a derivative row
@@ -356,10 +358,8 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
                 r[R_X] = minimum_image_fast(xi - r[R_X], Lx, P.invLx);
                 r[R_Y] = minimum_image_fast(yi - r[R_Y], Ly, P.invLy);
                 r[R_RMAX] = lim * lim;
-                if constexpr (!USER) {
-                    const int wj = unpack_w(r[R_W]);
-                    r[R_W] = P.cA[(wj >> 3) == pi ? 1 : 0][ti][wj & 7];
-                }
+                const int wj = unpack_w(r[R_W]);
+                r[COUPLING] = P.cA[(wj >> 3) == pi ? 1 : 0][ti][wj & 7];
             }
         }
         __syncwarp();
@@ -521,7 +521,7 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
                     while (hm) {
                         int bit[2], sl[2];
                         const T* r[2];
-                        T dx[2], dy[2], gv[2];
+                        T dx[2], dy[2], dd[2], gv[2];
                         bit[0] = __ffsll((long long)hm) - 1;
                         hm &= hm - 1;
                         const bool two = hm != 0;
@@ -550,17 +550,14 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
                             const bool off = d2 >= T(2.2250738585072014e-308);
                             const T inv = rsqrt_normal(off ? d2 : T(1));
                             const T dist = off ? d2 * inv : T(0);
-                            const T dd = radius_at64(r[i], off ? dx[i] * inv : T(1), off ? dy[i] * inv : T(0)) - dist;
+                            dd[i] = radius_at64(r[i], off ? dx[i] * inv : T(1), off ? dy[i] * inv : T(0)) - dist;
                             // pair coupling of the terms (src/energies/contact.jl:267-293)
-                            if constexpr (USER) {
-                                const int wj = unpack_w(r[i][R_W]);
-                                gv[i] = dd >= T(0) ? P.cA[(wj >> 3) == pi ? 1 : 0][ti][wj & 7] : T(0);
-                                if (dd > T(0)) gv[i] += P.cB[ti] * dd;
-                                gv[i] += user_pressure(P, dd, ti, wj, pi);
-                            } else {
-                                gv[i] = dd >= T(0) ? r[i][R_W] : T(0);
-                                gv[i] = dd > T(0) ? fma(cB, dd, gv[i]) : gv[i];
-                            }
+                            gv[i] = dd[i] >= T(0) ? r[i][COUPLING] : T(0);
+                            gv[i] = dd[i] > T(0) ? fma(cB, dd[i], gv[i]) : gv[i];
+                        }
+                        if constexpr (USER) {
+                            const int wj[2] = {unpack_w(r[0][R_W]), unpack_w(r[1][R_W])};
+                            user_pressure(P, dd, ti, wj, pi, gv);
                         }
                         wp[sl[0] * 32] += gv[0];
                         if (two) wp[sl[1] * 32] += gv[1];
@@ -583,18 +580,21 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
             GR[sl] = W * r * iq + pw * r;
             GD[sl] = W * r1 * iq;
             GDD[sl] = T(0);
-            if constexpr (USER)
-                if (v) ub.gradients(P, ti, r, r1, R2[sl], GR[sl], GD[sl], GDD[sl]);
             fx += pw * (r * e.x + r1 * e.y);
             fy += pw * (r * e.y - r1 * e.x);
             tt += (-pw * r) * r1;
-            if (MODE == MODE_DIAG && act && v) {
-                const size_t o = (size_t)g * nth + k;
-                d.P[o] = p;
-                d.GR[o] = GR[sl];
-                d.GD[o] = GD[sl];
-                d.GDD[o] = GDD[sl];
-            }
+            if (MODE == MODE_DIAG && act && v) d.P[(size_t)g * nth + k] = p;
+        }
+        if constexpr (USER) ub.gradients(P, ti, vmask, R, R1, R2, GR, GD, GDD);
+        if (MODE == MODE_DIAG && act) {
+#pragma unroll
+            for (int sl = 0; sl < S; ++sl)
+                if (vmask & (1u << sl)) {
+                    const size_t o = (size_t)g * nth + k0 + l + 8 * sl;
+                    d.GR[o] = GR[sl];
+                    d.GD[o] = GD[sl];
+                    d.GDD[o] = GDD[sl];
+                }
         }
         // pullback of the chunk
         const int c = lane >> 2;

@@ -1304,14 +1304,19 @@ struct UserBody {
 #pragma unroll
             for (int j = 0; j < fcc_user::MAX_M; ++j) Q[u][j] = T(0);
             if (!on(P, u, ti)) continue;
-#pragma unroll
-            for (int sl = 0; sl < S; ++sl)
-                if (vmask & (1u << sl)) {
-                    T q[fcc_user::MAX_M] = {};
-                    fcc_user::body_q<T>(P.ub_id[u], R[sl], R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], q);
-#pragma unroll
-                    for (int j = 0; j < fcc_user::MAX_M; ++j) Q[u][j] += q[j];
-                }
+            // one branch per term, then the nodes side by side (a node beyond
+            // the contour as a unit circle's, its value dropped)
+#define FCC_UT_CASE(i, F)                                                                                    \
+    if (P.ub_id[u] == i) {                                                                                   \
+        _Pragma("unroll") for (int sl = 0; sl < S; ++sl) {                                                   \
+            const bool v = vmask & (1u << sl);                                                               \
+            T q[fcc_user::MAX_M] = {};                                                                       \
+            fcc_user::F::q(v ? R[sl] : T(1), R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], q);                       \
+            _Pragma("unroll") for (int j = 0; j < fcc_user::MAX_M; ++j) Q[u][j] += v ? q[j] : T(0);          \
+        }                                                                                                    \
+    }
+            FCC_USER_BODY_TERMS(FCC_UT_CASE)
+#undef FCC_UT_CASE
         }
         // every lane of the warp takes the shuffles (a warp may hold bodies of several types)
 #pragma unroll
@@ -1334,32 +1339,49 @@ struct UserBody {
             E += fcc_user::body_F<T>(P.ub_id[u], Q[u], r0, ti + 1, P.ub_a[u], P.ub_b[u]);
         }
     }
-    __device__ __forceinline__ void gradients(const SimDesc<T>& P, int ti, T r, T r1, T r2, T& GR, T& GD, T& GDD) const {
+    template <int S>
+    __device__ __forceinline__ void gradients(const SimDesc<T>& P, int ti, unsigned vmask, const T (&R)[S],
+                                              const T (&R1)[S], const T (&R2)[S], T (&GR)[S], T (&GD)[S],
+                                              T (&GDD)[S]) const {
 #pragma unroll
         for (int u = 0; u < MUT; ++u) {
             if (!on(P, u, ti)) continue;
-            T dq[fcc_user::MAX_M][3] = {};
-            fcc_user::body_dq<T>(P.ub_id[u], r, r1, r2, P.ub_a[u], P.ub_b[u], dq);
-#pragma unroll
-            for (int j = 0; j < fcc_user::MAX_M; ++j) {
-                GR += w[u][j] * dq[j][0];
-                GD += w[u][j] * dq[j][1];
-                GDD += w[u][j] * dq[j][2];
-            }
+#define FCC_UT_CASE(i, F)                                                                                    \
+    if (P.ub_id[u] == i) {                                                                                   \
+        _Pragma("unroll") for (int sl = 0; sl < S; ++sl) {                                                   \
+            const bool v = vmask & (1u << sl);                                                               \
+            T dq[fcc_user::MAX_M][3] = {};                                                                   \
+            fcc_user::F::dq(v ? R[sl] : T(1), R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], dq);                     \
+            _Pragma("unroll") for (int j = 0; j < fcc_user::MAX_M; ++j) {                                    \
+                const T wj = v ? w[u][j] : T(0);                                                             \
+                GR[sl] += wj * dq[j][0];                                                                     \
+                GD[sl] += wj * dq[j][1];                                                                     \
+                GDD[sl] += wj * dq[j][2];                                                                    \
+            }                                                                                                \
+        }                                                                                                    \
+    }
+            FCC_USER_BODY_TERMS(FCC_UT_CASE)
+#undef FCC_UT_CASE
         }
     }
 };
 
-// Pressure of the user contact terms at depth dd against a body with record
-// word wj.
-template <class T>
-__device__ __forceinline__ T user_pressure(const SimDesc<T>& P, T dd, int ti, int wj, int pi) {
-    T gv = T(0);
+// Pressures of the user contact terms at the depths dd of H hits against
+// bodies with record words wj, added to gv.
+template <int H, class T>
+__device__ __forceinline__ void user_pressure(const SimDesc<T>& P, const T (&dd)[H], int ti, const int (&wj)[H], int pi,
+                                              T (&gv)[H]) {
 #pragma unroll
-    for (int u = 0; u < MUT; ++u)
-        if (u < P.nuc && ((P.uc_mask[u] >> ti) & 1u))
-            gv += fcc_user::contact_g<T>(P.uc_id[u], dd, ti + 1, (wj & 7) + 1, (wj >> 3) == pi, P.uc_a[u], P.uc_b[u]);
-    return gv;
+    for (int u = 0; u < MUT; ++u) {
+        if (u >= P.nuc || !((P.uc_mask[u] >> ti) & 1u)) continue;
+#define FCC_UT_CASE(i, F)                                                                                          \
+    if (P.uc_id[u] == i) {                                                                                         \
+        _Pragma("unroll") for (int k = 0; k < H; ++k) gv[k] +=                                                     \
+            fcc_user::F::g(dd[k], ti + 1, (wj[k] & 7) + 1, (wj[k] >> 3) == pi, P.uc_a[u], P.uc_b[u]);              \
+    }
+        FCC_USER_CONTACT_TERMS(FCC_UT_CASE)
+#undef FCC_UT_CASE
+    }
 }
 
 // Bond forces on the centre of body g (src/energies/bonds.jl:98-111), by
@@ -2647,9 +2669,12 @@ __global__ void k_finish_rebuild(DevPtrs<T> d) {
 // bodies' coefficient rows through shared memory with consecutive threads
 // reading consecutive doubles, so host reads cross PCIe in full lines.
 // ix_in, iy_in (image counters; null: keep the device's) likewise.
-// Launch with INIT_BLOCK threads and init_smem_bytes(in_nc) bytes.
-constexpr int INIT_BLOCK = 256;
-__host__ __device__ constexpr size_t init_smem_bytes(int in_nc) { return (size_t)INIT_BLOCK * in_nc * sizeof(double); }
+// Launch with INIT_BLOCK threads and init_smem_bytes(in_nc) bytes for every
+// INIT_BODIES bodies: every host read of a block is in flight at once, one
+// round trip over PCIe (256 bodies and threads per block took one for every
+// few of 19 reads: N = 1024 24 us, now 9).
+constexpr int INIT_BLOCK = 128, INIT_BODIES = 32;
+__host__ __device__ constexpr size_t init_smem_bytes(int in_nc) { return (size_t)INIT_BODIES * in_nc * sizeof(double); }
 template <class T>
 __global__ void __launch_bounds__(INIT_BLOCK) k_init(DevPtrs<T> d, int par, int g0, int n, const double* __restrict__ x,
                                                     const double* __restrict__ y, const double* __restrict__ th_in,
@@ -2657,15 +2682,29 @@ __global__ void __launch_bounds__(INIT_BLOCK) k_init(DevPtrs<T> d, int par, int 
                                                     const int* __restrict__ w, const int* __restrict__ ix_in,
                                                     const int* __restrict__ iy_in) {
     extern __shared__ double s_coef[];
-    const int i0 = blockIdx.x * INIT_BLOCK;
-    const int nb = min(INIT_BLOCK, n - i0);
-    for (int u = threadIdx.x; u < nb * in_nc; u += INIT_BLOCK) s_coef[u] = coef_in[(size_t)i0 * in_nc + u];
-    __syncthreads();
+    const int i0 = blockIdx.x * INIT_BODIES;
+    const int nb = min(INIT_BODIES, n - i0);
     const int i = i0 + threadIdx.x;
-    if (i >= n) return;
+    const bool own = threadIdx.x < nb;
+    constexpr int PER = (INIT_BODIES * NCM + INIT_BLOCK - 1) / INIT_BLOCK;
+    double cv[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int u = threadIdx.x + k * INIT_BLOCK;
+        cv[k] = u < nb * in_nc ? coef_in[(size_t)i0 * in_nc + u] : 0.0;
+    }
+    const double x_i = own ? x[i] : 0.0, y_i = own ? y[i] : 0.0, t_i = own ? th_in[i] : 0.0;
+    const int ix_i = own && ix_in ? ix_in[i] : 0, iy_i = own && iy_in ? iy_in[i] : 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int u = threadIdx.x + k * INIT_BLOCK;
+        if (u < nb * in_nc) s_coef[u] = cv[k];
+    }
+    __syncthreads();
+    if (!own) return;
     const int g = g0 + i;
-    if (ix_in) d.imgx[g] = ix_in[i];
-    if (iy_in) d.imgy[g] = iy_in[i];
+    if (ix_in) d.imgx[g] = ix_i;
+    if (iy_in) d.imgy[g] = iy_i;
     const int s = d.sim_of[g];
     const SimDesc<T>& P = d.sims[s];
     const int K = P.K;
@@ -2679,7 +2718,7 @@ __global__ void __launch_bounds__(INIT_BLOCK) k_init(DevPtrs<T> d, int par, int 
         c[1 + m] = m < kt ? T(ci[1 + m]) : T(0);
         c[1 + KM + m] = m < kt ? T(ci[1 + in_K + m]) : T(0);
     }
-    const T th_i = T(th_in[i]);
+    const T th_i = T(t_i);
     // enforce_shape! and the lab frame with the arithmetic of the update's
     // end of step (update_body): modes spread over 8 lanes as m = lane + 8u,
     // per-lane sums in u order, lanes combined by the xor butterfly of
@@ -2747,8 +2786,8 @@ __global__ void __launch_bounds__(INIT_BLOCK) k_init(DevPtrs<T> d, int par, int 
         bpl[l] = bp;
     }
     const T bound = c[0] + tree8(bpl);
-    rn[R_X] = T(x[i]);
-    rn[R_Y] = T(y[i]);
+    rn[R_X] = T(x_i);
+    rn[R_Y] = T(y_i);
     rn[R_RMAX] = r0 * bound;
     rn[R_A0] = r0 * c[0];
     T* tag = nullptr;
@@ -2900,37 +2939,48 @@ __global__ void k_geometry(DevPtrs<T> d, int par, T* lab, T* labR0, T* R, T* dR,
 }
 
 // perimeters, areas, shape index with FP64 node sums (src/observables.jl:7-18).
-// Bodies g0 .. g0+n-1, out indexed from g0.
+// Bodies g0 .. g0+n-1, out indexed from g0 (device memory, or page-locked host
+// memory written in place).  8 lanes per body, lane l the nodes l + 8 s: one
+// thread per body took 11 us at any size, 40 nodes of a recurrence in a row.
+constexpr int OBS_LANES = 8, OBS_BLOCK = 256;
 template <class T>
 __global__ void k_observables(DevPtrs<T> d, int par, int g0, int n, double* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    constexpr int L = OBS_LANES;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, l = t % L;
+    const int i = min(t / L, n - 1);  // every lane takes the shuffles
     const int g = g0 + i;
     const int s = d.sim_of[g];
-    if (s < 0) return;
+    if (s < 0) return;  // a slot's bodies are real: uniform over the grid
     const SimDesc<T>& P = d.sims[s];
     const T* rc = rec_cur(d, par) + (size_t)g * RECW;
+    T al[KM], be[KM];
+#pragma unroll
+    for (int m = 0; m < KM; ++m) al[m] = rc[r_al(m)], be[m] = rc[r_be(m)];
+    const T a0 = rc[R_A0];
     double per = 0.0, area = 0.0;
-    for (int k = 0; k < P.nth; ++k) {
+    for (int k = l; k < P.nth; k += L) {
         const T c1 = d.cs[2 * k], s1 = d.cs[2 * k + 1];
-        T c = c1, sn = s1, r = rc[R_A0], r1 = T(0);
+        T c = c1, sn = s1, r = a0, r1 = T(0);
+#pragma unroll
         for (int m = 0; m < KM; ++m) {
             const T n = T(m + 2);
             const T cn = c * c1 - sn * s1;
             sn = sn * c1 + c * s1;
             c = cn;
-            const T al = rc[r_al(m)], be = rc[r_be(m)];
-            r += al * c + be * sn;
-            r1 += n * (be * c - al * sn);
+            r += al[m] * c + be[m] * sn;
+            r1 += n * (be[m] * c - al[m] * sn);
         }
         per += sqrt((double)r * r + (double)r1 * r1);
         area += (double)r * r;
     }
-    per *= (double)P.dphi;
-    area *= (double)P.dphi / 2.0;
-    out[3 * (size_t)i] = per;
-    out[3 * (size_t)i + 1] = area;
-    out[3 * (size_t)i + 2] = per / sqrt(area);
+    per = group_sum<L>(per) * (double)P.dphi;
+    area = group_sum<L>(area) * ((double)P.dphi / 2.0);
+    // the block's results leave it in whole lines
+    __shared__ double s_out[3 * OBS_BLOCK / L];
+    if (l < 3) s_out[3 * (threadIdx.x / L) + l] = l == 0 ? per : l == 1 ? area : per / sqrt(area);
+    __syncthreads();
+    const int i0 = blockIdx.x * (OBS_BLOCK / L), nb = min(OBS_BLOCK / L, n - i0);
+    if (threadIdx.x < 3 * nb) out[3 * (size_t)i0 + threadIdx.x] = s_out[threadIdx.x];
 }
 
 // philox_noise! (src/random.jl:113-130): first three normals of body i.

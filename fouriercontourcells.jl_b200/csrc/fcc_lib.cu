@@ -141,13 +141,13 @@ V* mapped_view(V* p) {
     return static_cast<V*>(a.devicePointer);
 }
 
-// Device output of k_observables and its pinned host copy, grown on demand
-// and reused: an observable query allocates nothing after the first at its
-// size (allocation and release of device memory synchronise the device and
-// cost milliseconds).
+// Page-locked output of k_observables, which writes it in place, grown on
+// demand and reused: an observable query allocates nothing after the first at
+// its size (allocation and release synchronise the device and cost
+// milliseconds).
 struct ObsArea {
-    DBuf<double> dev;
     double* host = nullptr;
+    double* dev = nullptr;  // the device's address of it
     size_t cap = 0;
     ObsArea() = default;
     ObsArea(const ObsArea&) = delete;
@@ -155,13 +155,14 @@ struct ObsArea {
     ~ObsArea() {
         if (host) cudaFreeHost(host);
     }
-    fcc_status reserve(size_t n, cudaStream_t st) {
+    fcc_status reserve(size_t n) {
         if (n <= cap) return FCC_OK;
         if (host) cudaFreeHost(host);
         host = nullptr;
         cap = 0;
-        FCC_TRY(dev.alloc(n, st));
         CUDA_TRY(cudaMallocHost(&host, n * sizeof(double)));
+        dev = mapped_view(host);
+        if (!dev) return fail(FCC_ERR_UNSUPPORTED, "page-locked memory is not mapped");
         cap = n;
         return FCC_OK;
     }
@@ -1001,7 +1002,7 @@ struct Engine final : EngineBase {
         }
         const DevPtrs<T> d = ptrs();
         if (N > 0) {
-            const int grid = (int)((N + INIT_BLOCK - 1) / INIT_BLOCK);
+            const int grid = (int)((N + INIT_BODIES - 1) / INIT_BODIES);
             k_init<T><<<grid, INIT_BLOCK, init_smem_bytes(nc), stream>>>(d, par(), 0, (int)N, px, py, pth, pc, nc, K,
                                                                         w_dev.p, pix, piy);
             CUDA_TRY(cudaGetLastError());
@@ -1420,10 +1421,9 @@ struct Engine final : EngineBase {
     fcc_status observable(int which, int32_t typ, double* out, int64_t* count) override {
         const double* v = nullptr;
         if (N > 0) {
-            FCC_TRY(obs.reserve(3 * (size_t)N, stream));
-            k_observables<T><<<(int)((N + 127) / 128), 128, 0, stream>>>(ptrs(), par(), 0, (int)N, obs.dev.p);
+            FCC_TRY(obs.reserve(3 * (size_t)N));
+            k_observables<T><<<(int)((N * OBS_LANES + OBS_BLOCK - 1) / OBS_BLOCK), OBS_BLOCK, 0, stream>>>(ptrs(), par(), 0, (int)N, obs.dev);
             CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaMemcpyAsync(obs.host, obs.dev.p, 3 * (size_t)N * sizeof(double), cudaMemcpyDeviceToHost, stream));
             FCC_TRY(sync_stream());
             v = obs.host;
         }

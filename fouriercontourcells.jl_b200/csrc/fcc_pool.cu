@@ -534,7 +534,7 @@ struct Pool final : PoolBase {
         CUDA_TRY(cudaMemcpyAsync(dx + 3 * n, b->coef, n * P.nc * sizeof(double), cudaMemcpyHostToDevice, stream));
         FCC_TRY(st_w.upload(w, stream));
         const DevPtrs<T> d = ptrs();
-        const int blocks = (int)((n + INIT_BLOCK - 1) / INIT_BLOCK);
+        const int blocks = (int)((n + INIT_BODIES - 1) / INIT_BODIES);
         k_init<T><<<blocks, INIT_BLOCK, init_smem_bytes(P.nc), stream>>>(d, par(), (int)S.off, (int)n, dx, dx + n,
                                                                           dx + 2 * n, dx + 3 * n, P.nc, P.K, st_w.p(),
                                                                           nullptr, nullptr);
@@ -1069,10 +1069,9 @@ struct Pool final : PoolBase {
         const int64_t N = S.spec.N;
         const double* v = nullptr;
         if (N > 0) {
-            FCC_TRY(obs.reserve(3 * (size_t)N, stream));
-            k_observables<T><<<(int)((N + 127) / 128), 128, 0, stream>>>(ptrs(), par(), (int)S.off, (int)N, obs.dev.p);
+            FCC_TRY(obs.reserve(3 * (size_t)N));
+            k_observables<T><<<(int)((N * OBS_LANES + OBS_BLOCK - 1) / OBS_BLOCK), OBS_BLOCK, 0, stream>>>(ptrs(), par(), (int)S.off, (int)N, obs.dev);
             CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cudaMemcpyAsync(obs.host, obs.dev.p, 3 * (size_t)N * sizeof(double), cudaMemcpyDeviceToHost, stream));
             FCC_TRY(sync_stream());
             v = obs.host;
         }

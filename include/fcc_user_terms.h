@@ -44,7 +44,23 @@
 #define FCC_HD inline
 #endif
 
+#if defined(__CUDACC__)
+namespace fcc {
+__device__ __forceinline__ double rsqrt_normal(double x);
+}
+#endif
+
 namespace fcc_user {
+
+/* 1 / sqrt(x) for x > 0 in FP64: without the branches of sqrt and of a
+ * division on the device, so that a term's nodes overlap. */
+FCC_HD double inv_sqrt(double x) {
+#if defined(__CUDA_ARCH__)
+    return fcc::rsqrt_normal(x);
+#else
+    return 1.0 / sqrt(x);
+#endif
+}
 
 /* Bending energy kappa * contour integral of c^2 ds, kappa = a: the
  * reference README's example of an integrand-only body term
@@ -54,13 +70,24 @@ struct Bending {
     template <class T>
     FCC_HD static void q(T R, T dR, T ddR, T a, T, T* out) {
         const T S = R * R + dR * dR, N = R * R + T(2) * dR * dR - R * ddR;
-        out[0] = a * N * N / (S * S * sqrt(S));
+        if constexpr (sizeof(T) == 8) {
+            const T r = inv_sqrt(S), r2 = r * r;
+            out[0] = a * N * N * (r2 * r2 * r);
+        } else {
+            out[0] = a * N * N / (S * S * sqrt(S));
+        }
     }
     template <class T>
     FCC_HD static void dq(T R, T dR, T ddR, T a, T, T (*out)[3]) {
         // q = a N^2 S^(-5/2):  dq/dx = a N S^(-7/2) (2 S dN/dx - 5/2 N dS/dx)
         const T S = R * R + dR * dR, N = R * R + T(2) * dR * dR - R * ddR;
-        const T f = a * N / (S * S * S * sqrt(S));
+        T f;
+        if constexpr (sizeof(T) == 8) {
+            const T r = inv_sqrt(S), r2 = r * r;
+            f = a * N * (r2 * r2 * r2 * r);
+        } else {
+            f = a * N / (S * S * S * sqrt(S));
+        }
         out[0][0] = f * (T(2) * S * (T(2) * R - ddR) - T(5) * N * R);
         out[0][1] = f * (T(8) * S * dR - T(5) * N * dR);
         out[0][2] = f * (-T(2) * S * R);
@@ -80,14 +107,21 @@ struct ShapeIndexElasticity {
     static constexpr int M = 2;
     template <class T>
     FCC_HD static void q(T R, T dR, T, T, T, T* out) {
-        out[0] = sqrt(R * R + dR * dR);
+        if constexpr (sizeof(T) == 8) out[0] = (R * R + dR * dR) * inv_sqrt(R * R + dR * dR);
+        else out[0] = sqrt(R * R + dR * dR);
         out[1] = R * R / T(2);
     }
     template <class T>
     FCC_HD static void dq(T R, T dR, T, T, T, T (*out)[3]) {
-        const T s = sqrt(R * R + dR * dR);
-        out[0][0] = R / s;
-        out[0][1] = dR / s;
+        if constexpr (sizeof(T) == 8) {
+            const T r = inv_sqrt(R * R + dR * dR);
+            out[0][0] = R * r;
+            out[0][1] = dR * r;
+        } else {
+            const T s = sqrt(R * R + dR * dR);
+            out[0][0] = R / s;
+            out[0][1] = dR / s;
+        }
         out[0][2] = T(0);
         out[1][0] = R;
         out[1][1] = T(0);
