@@ -358,6 +358,9 @@ __device__ WorkList build_worklist(const DevPtrs<T>& d, int* area, int cap) {
     return w;
 }
 
+// cells per range total of a lone simulation's scan
+constexpr int SCAN_RANGE = 512;
+
 template <class T>
 __device__ __forceinline__ void count_body(const DevPtrs<T>& d, const SimDesc<T>& P, int par, int g) {
     const T* r = rec_cur(d, par) + (size_t)g * RECW;
@@ -366,6 +369,11 @@ __device__ __forceinline__ void count_body(const DevPtrs<T>& d, const SimDesc<T>
     const int cell = P.cell_off + cx + P.ncx * cy;
     d.cellid[g] = cell;
     d.slot[g] = atomicAdd(&d.ccount[cell], 1);
+    if (d.ctot) {  // a warp's bodies share few ranges: one addition for each
+        const int r = cell / SCAN_RANGE;
+        const unsigned same = __match_any_sync(__activemask(), r);
+        if ((threadIdx.x & 31) == __ffs((int)same) - 1) atomicAdd(&d.ctot[r], __popc(same));
+    }
 }
 
 // `lone_need`: a single simulation's rebuild decision as the block knows it
@@ -465,6 +473,8 @@ __device__ void phase_scatter(const DevPtrs<T>& d, int tid, int nthr, const Work
         }
         return;
     }
+    if (d.ctot && (ldcg(d.flags) & F_NEED))  // the totals are read for the last time in the scan
+        for (int r = tid; r * SCAN_RANGE < d.Ctot; r += nthr) d.ctot[r] = 0;
     for (int g = tid; g < d.Ntot; g += nthr) {
         const int s = __ldg(d.sim_of + g);
         if (s < 0 || !(ldcg(d.flags + s) & F_NEED)) continue;
@@ -566,9 +576,8 @@ __device__ void phase_neighbors(const DevPtrs<T>& d, int par, int tid, int nthr,
         T xi = T(0), yi = T(0), rmi = T(0), ri = T(0);
         int qa0 = 0, cnt0 = 0, qa8 = 0, cnt8 = 0;
         if (act) {
-            xi = ldcg(rc + (size_t)g * RECW + R_X);
-            yi = ldcg(rc + (size_t)g * RECW + R_Y);
-            rmi = ldcg(rc + (size_t)g * RECW + R_RMAX);
+            T wi;
+            load_head(rc + (size_t)g * RECW, xi, yi, rmi, wi);
             ri = add_rn(rmi, P->nbrange);
             int cx, cy;
             grid_coords(*P, xi, yi, cx, cy);
@@ -625,8 +634,8 @@ __device__ void phase_neighbors(const DevPtrs<T>& d, int par, int tid, int nthr,
 #pragma unroll
             for (int i = 0; i < NB_PER; ++i) {
                 if (j[i] >= 0 && j[i] != g) {
-                    const T* rj = rc + (size_t)j[i] * RECW;
-                    const T xj = ldcg(rj + R_X), yj = ldcg(rj + R_Y), rmj = ldcg(rj + R_RMAX);
+                    T xj, yj, rmj, wj;
+                    load_head(rc + (size_t)j[i] * RECW, xj, yj, rmj, wj);
                     const T dx = minimum_image_exact(sub_rn(xi, xj), P->Lx);
                     const T dy = minimum_image_exact(sub_rn(yi, yj), P->Ly);
                     const T lim = add_rn(ri, rmj);

@@ -102,6 +102,10 @@ struct DBuf {
     }
 };
 
+// ranges of a lone simulation's cell scan, and blocks that take them
+inline size_t scan_ranges(size_t cells) { return (cells + SCAN_RANGE - 1) / SCAN_RANGE; }
+inline int scan_grid(int64_t cells) { return (int)std::min<size_t>(scan_ranges((size_t)cells), 148 * 8); }
+
 // blocks of 256 threads for the neighbour phase (8 lanes per body), capped;
 // the phase loops over the rest
 inline int neighbor_grid(int64_t n) { return (int)std::min<int64_t>((n + 31) / 32, 148 * 64); }
@@ -717,6 +721,7 @@ struct Engine final : EngineBase {
         d.cstart = cstart.p;
         d.cstop = cstop.p;
         d.ccount = ccount.p;
+        d.ctot = ccount.p + (size_t)ncx * ncy;
         d.cell_sim = cell_sim.p;
         d.ccap = ccap;
         d.ch_idx = ch_idx.p;
@@ -820,7 +825,7 @@ struct Engine final : EngineBase {
         FCC_TRY(perm.alloc(n, stream));
         FCC_TRY(cstart.alloc((size_t)ncx * ncy, stream));
         FCC_TRY(cstop.alloc((size_t)ncx * ncy, stream));
-        FCC_TRY(ccount.alloc((size_t)ncx * ncy, stream));
+        FCC_TRY(ccount.alloc((size_t)ncx * ncy + scan_ranges((size_t)ncx * ncy), stream));  // counts, then range totals
         FCC_TRY(cell_sim.alloc((size_t)ncx * ncy, stream));
         FCC_TRY(ch_idx.upload(chi, stream));
         FCC_TRY(ch_count.upload(chc, stream));
@@ -1145,7 +1150,7 @@ struct Engine final : EngineBase {
             }
             k_prepare_rebuild<T><<<1, 256, 0, stream>>>(dd, (force || attempt > 0) ? 1 : 0);
             k_phase_count<T><<<grid, 256, 0, stream>>>(dd, par());
-            k_phase_scan<T><<<1, 1024, 0, stream>>>(dd);
+            k_phase_scan<T><<<scan_grid(ncx * ncy), 256, 0, stream>>>(dd);
             k_phase_scatter<T><<<grid, 256, 0, stream>>>(dd);
             k_phase_sort<T><<<(ncx * ncy + 255) / 256, 256, 0, stream>>>(dd);
             k_phase_neighbors<T><<<neighbor_grid(N), 256, 0, stream>>>(dd, par());
@@ -1508,8 +1513,9 @@ struct ListWork {
             for (DBuf<int>* b : {&sim_of, &cellid, &slot, &perm, &nb_count}) FCC_TRY(b->alloc(n_, st));
             n = n_;
         }
-        if (cells_ > cells) {  // ccount is zero between builds (phase_scan clears it)
-            for (DBuf<int>* b : {&cstart, &cstop, &ccount, &cell_sim}) FCC_TRY(b->alloc(cells_, st));
+        if (cells_ > cells) {  // counts and totals are zero between builds (the phases clear them)
+            for (DBuf<int>* b : {&cstart, &cstop, &cell_sim}) FCC_TRY(b->alloc(cells_, st));
+            FCC_TRY(ccount.alloc(cells_ + scan_ranges(cells_), st));  // counts, then range totals
             cells = cells_;
         }
         if (ids_ > ids) {
@@ -1624,6 +1630,7 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
     d.cstart = w->cstart.p;
     d.cstop = w->cstop.p;
     d.ccount = w->ccount.p;
+    d.ctot = w->ccount.p + w->cells;
     d.cell_sim = w->cell_sim.p;
     d.nb_idx = w->nb_idx.p;
     d.nb_count = w->nb_count.p;
@@ -1635,7 +1642,7 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
     const int grid = (int)((N + 255) / 256);
     k_pack_head<T><<<grid, 256, 0, st>>>(d.rec0, xd, yd, rd, (int)N);
     k_phase_count<T><<<grid, 256, 0, st>>>(d, 0);
-    k_phase_scan<T><<<1, 1024, 0, st>>>(d);
+    k_phase_scan<T><<<scan_grid((int64_t)C), 256, 0, st>>>(d);
     k_phase_scatter<T><<<grid, 256, 0, st>>>(d);
     k_phase_sort<T><<<(int)((C + 255) / 256), 256, 0, st>>>(d);
     k_phase_neighbors<T><<<neighbor_grid(N), 256, 0, st>>>(d, 0);

@@ -102,3 +102,29 @@ def test_neighbor_workspace_over_sizes_precisions_and_threads():
     with pytest.raises(fcc.ArgumentError):
         fcc.build_neighbors(*jobs[0][0][:5], -1.0, 0.3)
     same(fcc.build_neighbors(*jobs[0][0], **jobs[0][1]), want[0])
+
+
+@pytest.mark.parametrize("nx,ny,n", [(3, 3, 5), (7, 73, 200), (16, 32, 4000), (27, 19, 300), (32, 32, 1), (33, 31, 3000),
+                                     (200, 190, 50), (171, 180, 30000)])
+def test_cell_scan_over_its_ranges(nx, ny, n):
+    """Grids of fewer, exactly and more cells than one range of the scan (512),
+    densely and sparsely filled: cell lists and neighbour lists equal the
+    oracle's, in a build of its own and inside the step kernel."""
+    rng = np.random.default_rng(nx * ny + n)
+    cutoff = 3.2
+    Lx, Ly = nx * cutoff * 1.0001, ny * cutoff * 1.0001
+    x, y = rng.random(n) * Lx, rng.random(n) * Ly
+    same(fcc.build_neighbors(x, y, np.full(n, 1.1), Lx, Ly, cutoff, 0.3, cap=64),
+         oracle.build_neighbors(x, y, np.full(n, 1.1), Lx, Ly, cutoff, 0.3, cap=64))
+    R0 = (cutoff - 0.3) / (2 * (1 + np.sqrt(2 / 3)))  # the radius whose grid has this cutoff
+    coef = np.zeros((7, n), order="F")
+    coef[0] = 1.0
+    bodies = fcc.Bodies.new(x, y, np.zeros(n), coef, np.full(n, R0))
+    kw = dict(types=(fcc.BodyType(v0=0.5),), energies=(fcc.Overlap(0.1),), nθ=16, nl_capacity=64)
+    s, o = (cls(bodies, fcc.PeriodicBox(Lx, Ly), T=np.float64, **kw) for cls in (fcc.Simulation, oracle.OracleSimulation))
+    s.run(2)
+    o.step(2)
+    a, b = s.neighbors, o.neighbors
+    assert a.ncx * a.ncy == b.ncx * b.ncy and s.builds == o.builds
+    for f in ("cellid", "perm", "start", "stop", "count"):
+        assert np.array_equal(getattr(a, f), getattr(b, f)), f
