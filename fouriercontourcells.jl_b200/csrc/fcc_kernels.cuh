@@ -396,69 +396,116 @@ __device__ void phase_count(const DevPtrs<T>& d, int par, int tid, int nthr, con
     }
 }
 
-// exclusive scan of the cell counts of each flagged simulation (one block per
-// simulation); cell c holds perm[cstart[c] .. cstop[c]).  The cells go in
-// chunks of SCAN_PER per thread: a thread loads its run of counts into
-// registers (independent loads), one block-wide scan of the run totals gives
-// the run's first slot, and the thread writes its run from the registers.
-constexpr int SCAN_PER = 16;
-template <class T>
-__device__ void phase_scan(const DevPtrs<T>& d, const WorkList* wl) {
+// exclusive scan of cells [c0, c1) from the first slot `carry`, by one block:
+// cell c holds perm[cstart[c] .. cstop[c]), and the counts are cleared for the
+// next build.  The cells go in chunks of PER per thread: a thread loads its
+// run of counts into registers (independent loads), one block-wide scan of the
+// run totals gives the run's first slot, and the thread writes its run from
+// the registers, in 16-byte accesses where the run is whole and aligned.
+template <int PER, class T>
+__device__ __forceinline__ void scan_cells(const DevPtrs<T>& d, int c0, int c1, int carry) {
     __shared__ int s_warp[32];
     const int nw = (blockDim.x + 31) / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int base = c0; base < c1; base += blockDim.x * PER) {
+        const int u0 = base + threadIdx.x * PER;
+        int v[PER];
+        int sum = 0;
+        const bool whole = u0 + PER <= c1 && (u0 & 3) == 0;
+        if (whole) {
+#pragma unroll
+            for (int i = 0; i < PER; i += 4) {
+                const int4 q = __ldcg(reinterpret_cast<const int4*>(d.ccount + u0 + i));
+                v[i] = q.x, v[i + 1] = q.y, v[i + 2] = q.z, v[i + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) v[i] = u0 + i < c1 ? ldcg(d.ccount + u0 + i) : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) sum += v[i];
+        int incl = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += o;
+        }
+        if (lane == 31) s_warp[w] = incl;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            int t = threadIdx.x < nw ? s_warp[threadIdx.x] : 0;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, t, off);
+                if ((int)threadIdx.x >= off) t += o;
+            }
+            s_warp[threadIdx.x] = t;  // inclusive over warps
+        }
+        __syncthreads();
+        int st = carry + (w ? s_warp[w - 1] : 0) + incl - sum;
+        if (whole) {
+#pragma unroll
+            for (int i = 0; i < PER; i += 4) {
+                const int a = st, b = a + v[i], c = b + v[i + 1], e = c + v[i + 2];
+                st = e + v[i + 3];
+                *reinterpret_cast<int4*>(d.cstart + u0 + i) = make_int4(a, b, c, e);
+                *reinterpret_cast<int4*>(d.cstop + u0 + i) = make_int4(b, c, e, st);
+                *reinterpret_cast<int4*>(d.ccount + u0 + i) = make_int4(0, 0, 0, 0);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                if (u0 + i < c1) {
+                    d.cstart[u0 + i] = st;
+                    st += v[i];
+                    d.cstop[u0 + i] = st;
+                    d.ccount[u0 + i] = 0;
+                }
+            }
+        }
+        carry += s_warp[nw - 1];
+        __syncthreads();  // s_warp is rewritten by the next chunk
+    }
+}
+
+// Cell starts of every flagged simulation.  One simulation with range totals
+// (ctot, from the count phase): a block per range of SCAN_RANGE cells, which
+// first sums the totals before its own; the blocks clear no totals (others may
+// still read them: the scatter phase does).  Otherwise a block per
+// simulation.  (One block for the 57 000 cells of 262 144 bodies took 42 us of
+// a rebuild, for the 14 000 of 65 536 in a launch of its own 22 us.)
+template <class T>
+__device__ void phase_scan(const DevPtrs<T>& d, const WorkList* wl) {
+    auto built = [&](int s) {
+        d.builds[s] += 1;
+        d.maxcount[s] = 0;
+        atomicOr(&d.flags[s], F_VALID);
+    };
+    if (!wl && d.nsims == 1 && d.ctot) {
+        if (!(ldcg(d.flags) & F_NEED)) return;
+        const int nc = d.sims[0].ncells;
+        for (int r = blockIdx.x; r * SCAN_RANGE < nc; r += gridDim.x) {
+            __shared__ int s_before;
+            if (threadIdx.x == 0) s_before = 0;
+            __syncthreads();
+            int t = 0;
+            for (int q = threadIdx.x; q < r; q += blockDim.x) t += ldcg(d.ctot + q);
+            t = __reduce_add_sync(0xffffffffu, t);
+            if ((threadIdx.x & 31) == 0 && t) atomicAdd(&s_before, t);
+            __syncthreads();
+            const int before = s_before;
+            scan_cells<4>(d, r * SCAN_RANGE, min(nc, (r + 1) * SCAN_RANGE), before);
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) built(0);
+        return;
+    }
     const int nk = wl ? wl->m : d.nsims;
     for (int k = blockIdx.x; k < nk; k += gridDim.x) {
         const int s = wl ? wl->sim[k] : k;
         if (!wl && !(ldcg(d.flags + s) & F_NEED)) continue;
         const SimDesc<T>& P = d.sims[s];
-        int carry = P.body_off;
-        for (int base = 0; base < P.ncells; base += blockDim.x * SCAN_PER) {
-            const int u0 = base + threadIdx.x * SCAN_PER;
-            const int c0 = P.cell_off + u0;
-            int v[SCAN_PER];
-            int sum = 0;
-#pragma unroll
-            for (int i = 0; i < SCAN_PER; ++i) {
-                v[i] = u0 + i < P.ncells ? ldcg(d.ccount + c0 + i) : 0;
-                sum += v[i];
-            }
-            int incl = sum;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int o = __shfl_up_sync(0xffffffffu, incl, off);
-                if (lane >= off) incl += o;
-            }
-            if (lane == 31) s_warp[w] = incl;
-            __syncthreads();
-            if (threadIdx.x < 32) {
-                int t = threadIdx.x < nw ? s_warp[threadIdx.x] : 0;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int o = __shfl_up_sync(0xffffffffu, t, off);
-                    if ((int)threadIdx.x >= off) t += o;
-                }
-                s_warp[threadIdx.x] = t;  // inclusive over warps
-            }
-            __syncthreads();
-            int st = carry + (w ? s_warp[w - 1] : 0) + incl - sum;
-#pragma unroll
-            for (int i = 0; i < SCAN_PER; ++i) {
-                if (u0 + i < P.ncells) {
-                    d.cstart[c0 + i] = st;
-                    st += v[i];
-                    d.cstop[c0 + i] = st;
-                    d.ccount[c0 + i] = 0;
-                }
-            }
-            carry += s_warp[nw - 1];
-            __syncthreads();  // s_warp is rewritten by the next chunk
-        }
-        if (threadIdx.x == 0) {
-            d.builds[s] += 1;
-            d.maxcount[s] = 0;
-            atomicOr(&d.flags[s], F_VALID);
-        }
+        scan_cells<16>(d, P.cell_off, P.cell_off + P.ncells, P.body_off);
+        if (threadIdx.x == 0) built(s);
         __syncthreads();
     }
 }
@@ -2199,11 +2246,34 @@ __device__ __forceinline__ void draw_ahead(const DevPtrs<T>& d, int wg, T* stage
     ahead[32] = z1;
 }
 
+// What phase B of the split step needs of a body's own state: none of it
+// depends on other bodies' forces, so a warp loads it, and draws its noise,
+// while it waits at the barrier between the phases.
+template <class T, int L>
+struct SplitOwn {
+    T x, y, w, th, r0, nz[2];
+    UpdatePre<T, L> pre;
+};
+template <class T, int L>
+__device__ __forceinline__ void load_split_own(const DevPtrs<T>& d, const SimDesc<T>& P, int par, int gg, int l,
+                                               long long clk, SplitOwn<T, L>& o) {
+    const T* rec = rec_cur(d, par) + (size_t)gg * RECW;
+    T rmax;
+    load_head(rec, o.x, o.y, rmax, o.w);
+    o.th = ldcg(rec + R_TH);
+    o.r0 = __ldg(d.R0 + gg);
+    load_update_pre(d, gg, l, P.K, o.pre);
+    o.nz[0] = o.nz[1] = T(0);
+    if (P.has_noise)
+        philox_pair<T>(P.k0, P.k1, (uint32_t)(gg - P.body_off + 1), (uint64_t)clk, l == 1 ? 0u : 1u, o.nz[0], o.nz[1]);
+}
+
 // Phase B of the split step: displacement with parent drag + update of the
-// bodies of warp group `wg`, from the forces phase A stored.
+// bodies of warp group `wg`, from the forces phase A stored.  `ahead`: the
+// bodies' own state, already loaded (lone simulations), or null.
 template <class T, int L>
 __device__ __forceinline__ void update_warp_split(const DevPtrs<T>& d, int wg, int par, const SimDesc<T>* sim0,
-                                                  int* rbp) {
+                                                  int* rbp, const SplitOwn<T, L>* ahead) {
     constexpr int BPW = 32 / L;
     const int lane = threadIdx.x & 31;
     const int l = lane & (L - 1);
@@ -2220,24 +2290,27 @@ __device__ __forceinline__ void update_warp_split(const DevPtrs<T>& d, int wg, i
     const int fl = ldcg(d.flags + s);
     const bool act = valid && (fl & F_ACTIVE) && !(fl & (F_FROZEN | F_HOLD));
     const long long clk = ldcg(d.clock + s);
-    T rv[RECW];
-    load_rec(rec_cur(d, par) + (size_t)gg * RECW, rv);
-    if (valid && !act) carry_record<T, L>(d, g, l, par, rv);
-    T nz[2] = {T(0), T(0)};
-    if (P.has_noise)
-        philox_pair<T>(P.k0, P.k1, (uint32_t)(gg - P.body_off + 1), (uint64_t)clk, l == 1 ? 0u : 1u, nz[0], nz[1]);
-    const int ti = unpack_w(rv[R_W]) & 7;
-    const T r0 = __ldg(d.R0 + gg);
-    UpdatePre<T, L> pre;
-    load_update_pre(d, gg, l, P.K, pre);
-    T gl[NCM];
-#pragma unroll
-    for (int r = 0; r < NCM; ++r) gl[r] = ldcg(d.glab + (size_t)gg * NCM + r);
-    const T fx = ldcg(d.gx + gg), fy = ldcg(d.gy + gg), tt = ldcg(d.gth + gg);
+    if (valid && !act) {
+        T rv[RECW];
+        load_rec(rec_cur(d, par) + (size_t)gg * RECW, rv);
+        carry_record<T, L>(d, g, l, par, rv);
+    }
+    SplitOwn<T, L> own;
+    if (ahead) own = *ahead;
+    else load_split_own<T, L>(d, P, par, gg, l, clk, own);
+    const int ti = unpack_w(own.w) & 7;
+    // the lane's mode gradients and dE/da0 from the stored pullback
+    const T* gl = d.glab + (size_t)gg * NCM;
+    const T gl0 = ldcg(gl), fx = ldcg(d.gx + gg), fy = ldcg(d.gy + gg), tt = ldcg(d.gth + gg);
     T gA[UpdatePre<T, L>::MPL], gB[UpdatePre<T, L>::MPL];
-    lane_mode_grads<T, L>(gl, l, gA, gB);
-    update_body<T, L>(d, P, act, g, s, l, par, clk, rv[R_X], rv[R_Y], rv[R_W], rv[R_TH], r0, ti, fx, fy, tt, gl[0], gA,
-                      gB, pre, fl, nz, true, rbp);
+#pragma unroll
+    for (int u = 0; u < UpdatePre<T, L>::MPL; ++u) {
+        const int m = l + u * L;
+        gA[u] = m < KM ? ldcg(gl + 1 + m) : T(0);
+        gB[u] = m < KM ? ldcg(gl + 1 + KM + m) : T(0);
+    }
+    update_body<T, L>(d, P, act, g, s, l, par, clk, own.x, own.y, own.w, own.th, own.r0, ti, fx, fy, tt, gl0, gA, gB,
+                      own.pre, fl, own.nz, true, rbp);
 }
 
 template <class T>
@@ -2501,8 +2574,22 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
         }
         if (LAT) res.have = res.on;
         if (SPLIT) {
-            if (!grid_barrier(d.sync, bl, [](unsigned) { return -1; })) return;
-            for (int wg = g0 + warp; wg < g1; wg += WPB) update_warp_split<T, L>(d, wg, par, sim0, &bl.rebuild);
+            if (lone) {
+                SplitOwn<T, L> own;
+                const int first = g0 + warp;
+                const long long clk = bl.clock;
+                auto shadow = [&] {
+                    const int g = first * (32 / L) + (threadIdx.x & 31) / L;
+                    if (first < g1) load_split_own<T, L>(d, *sim0, par, g < d.Ntot ? g : 0, threadIdx.x & (L - 1), clk, own);
+                };
+                if (!flat_barrier(d.sync, bl, 0u, NoAfter{}, true, shadow)) return;
+                for (int wg = first; wg < g1; wg += WPB)
+                    update_warp_split<T, L>(d, wg, par, sim0, &bl.rebuild, wg == first ? &own : nullptr);
+            } else {
+                if (!grid_barrier(d.sync, bl, [](unsigned) { return -1; })) return;
+                for (int wg = g0 + warp; wg < g1; wg += WPB)
+                    update_warp_split<T, L>(d, wg, par, sim0, &bl.rebuild, nullptr);
+            }
         }
         const int f0 = bl.flags;  // fixed during the step (read before thread 0 may rewrite it)
         const long long c0 = bl.clock;

@@ -19,6 +19,7 @@
 #include <memory>
 #include <mutex>
 #include <set>
+#include <shared_mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -133,9 +134,37 @@ struct Stage {
 // writes in place (every page-locked allocation is mapped under unified
 // addressing), or null for any other pointer (pageable memory, device
 // memory, null).
+// Blocks of fcc_host_alloc are known by their ranges: their addresses are the
+// device's too, and looking them up costs 0.1 us where the runtime's query
+// takes 0.5 (a state exchange makes twelve).
+struct HostBlocks {
+    std::shared_mutex m;
+    std::map<uintptr_t, size_t> at;
+    static HostBlocks& all() {
+        static HostBlocks* b = new HostBlocks;
+        return *b;
+    }
+    void add(void* p, size_t n) {
+        std::unique_lock<std::shared_mutex> lk(m);
+        at[(uintptr_t)p] = n;
+    }
+    void drop(void* p) {
+        std::unique_lock<std::shared_mutex> lk(m);
+        at.erase((uintptr_t)p);
+    }
+    bool holds(const void* p) {
+        std::shared_lock<std::shared_mutex> lk(m);
+        auto it = at.upper_bound((uintptr_t)p);
+        if (it == at.begin()) return false;
+        --it;
+        return (uintptr_t)p < it->first + it->second;
+    }
+};
+
 template <class V>
 V* mapped_view(V* p) {
     if (!p) return nullptr;
+    if (HostBlocks::all().holds(p)) return p;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();  // not a pointer the runtime knows: not mapped
@@ -672,9 +701,14 @@ struct Engine final : EngineBase {
     GridSync* sync_d = nullptr;
     ObsArea obs;  // perimeters / areas / shape indices: reused device and pinned host buffers
     int ccap = 1, bcap = 1;
-    Status* st_h = nullptr;  // pinned read-back of the run state
-    Status* up_h = nullptr;  // pinned head written by load_state
-    LaunchStatus* ls_h = nullptr;  // pinned, written by the step kernel at the end of a launch
+    struct Pinned {
+        Status st, up;    // read-back of the run state; head written by load_state
+        LaunchStatus ls;  // written by the step kernel at the end of a launch
+    };
+    Pinned* pinned = nullptr;  // one page-locked block
+    Status* st_h = nullptr;
+    Status* up_h = nullptr;
+    LaunchStatus* ls_h = nullptr;
     LaunchStatus* ls_d = nullptr;  // the device's address of it
     long long ticket = 0;
     // state exchange with the host (set_state / get_state): the caller's
@@ -687,9 +721,7 @@ struct Engine final : EngineBase {
 
     ~Engine() override {
         if (stream) cudaStreamSynchronize(stream);
-        if (st_h) cudaFreeHost(st_h);
-        if (up_h) cudaFreeHost(up_h);
-        if (ls_h) cudaFreeHost(ls_h);
+        if (pinned) cudaFreeHost(pinned);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
@@ -763,10 +795,11 @@ struct Engine final : EngineBase {
         CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         CUDA_TRY(cudaEventCreate(&ev0));
         CUDA_TRY(cudaEventCreate(&ev1));
-        CUDA_TRY(cudaMallocHost(&st_h, sizeof(Status)));
-        CUDA_TRY(cudaMallocHost(&up_h, sizeof(Status)));
-        CUDA_TRY(cudaMallocHost(&ls_h, sizeof(LaunchStatus)));
-        *ls_h = LaunchStatus{};
+        CUDA_TRY(cudaMallocHost(&pinned, sizeof(Pinned)));
+        *pinned = Pinned{};
+        st_h = &pinned->st;
+        up_h = &pinned->up;
+        ls_h = &pinned->ls;
         ls_d = mapped_view(ls_h);
         if (!ls_d) return fail(FCC_ERR_UNSUPPORTED, "page-locked memory is not mapped");
 
@@ -1743,10 +1776,16 @@ fcc_status fcc_host_alloc(int64_t bytes, void** out) {
     *out = nullptr;
     if (bytes == 0) return FCC_OK;
     CUDA_TRY(cudaMallocHost(out, (size_t)bytes));
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, *out) == cudaSuccess && a.devicePointer == *out)
+        HostBlocks::all().add(*out, (size_t)bytes);
     return FCC_OK;
 }
 fcc_status fcc_host_free(void* ptr) {
-    if (ptr) CUDA_TRY(cudaFreeHost(ptr));
+    if (ptr) {
+        HostBlocks::all().drop(ptr);
+        CUDA_TRY(cudaFreeHost(ptr));
+    }
     return FCC_OK;
 }
 fcc_status fcc_get_gradients(fcc_sim* sim, const fcc_gradients_host* out) { SIM_CALL(get_gradients(out)); }
