@@ -5,8 +5,8 @@
 // the contour nodes l + 8 s, s < 5, of a chunk and the modes m = l (and lane
 // 0 m = 8 too).  The contractions over modes and nodes run on the FP64 tensor
 // cores (mma.sync m8n8k4, IEEE double products and sums):
-//   synthesis  [R_b ; R'_b] (8 rows) = [c_b ; c'_b] (8 x 20) . M^T (20 x 40)
-//   pullback   [g_b ; h_b]  (8 rows) = [GR_b ; GD_b] (8 x 40) . M (40 x 20)
+//   synthesis  [R_b ; R'_b] (8 rows) = [c_b ; c'_b] (8 x 20) . M^T (20 x 8 S)
+//   pullback   [g_b ; h_b]  (8 rows) = [GR_b ; GD_b] (8 x 8 S) . M (8 S x 20)
 // with rows 2b + h (b the body, h = bit 2 of the lane: value or derivative),
 // M[k] = (cos 2 phi_k, sin 2 phi_k, ..., cos 10 phi_k, sin 10 phi_k, 1, 0),
 // c the R0-scaled lab coefficients of the record and c' the derivative's
@@ -222,12 +222,12 @@ __device__ __forceinline__ void update_body64(const DevPtrs<double>& d, const Si
 // Forces on the 4 bodies of warp group `wg`, and in MODE_FUSED their update
 // (references: forces_warp).  `stage` is this warp's shared memory; `tab` the
 // block's copy of M and of the nodes' (cos, sin) (one chunk), else null.
-template <bool ONE, int MODE, bool USER, bool LAT>
+template <int S, bool ONE, int MODE, bool USER, bool LAT>
 __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, double* stage, int par,
                                               const SimDesc<double>* sim0, const double* tab, int* rbp,
                                               const BarrierLocal* lone, bool drawn, Resident<double, 8>* res) {
     typedef double T;
-    constexpr int L = 8, S = 5, BPW = 4;
+    constexpr int L = 8, BPW = 4;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int IDS = (NBMAX64 + L - 1) / L;
     constexpr int MPL = 2;  // modes per lane
@@ -259,7 +259,7 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
 
     // the matrix and the nodes' (cos, sin): in shared memory but for a contour of many chunks
     const T* mat = ONE || tab ? tab : d.basis;
-    const T* cst = ONE || tab ? tab + m64_rows(ONE) * M64_COLS : d.cs;
+    const T* cst = ONE || tab ? tab + m64_rows(ONE, S) * M64_COLS : d.cs;
 
     // ---- independent loads first
     const T* grec = rc + (size_t)gg * RECW;
@@ -372,7 +372,7 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
     const int ns = ONE ? S : (nth + 8 * nch - 1) / (8 * nch);
     T R[S], R1[S], R2[S];
     unsigned vmask = 0;
-    T fa[S];  // synthesis A fragment of this lane's row, one value per k-step
+    T fa[5];  // synthesis A fragment of this lane's row, one value per k-step
     auto load_row = [&]() {
         const T n0 = T((tq >> 1) + 2);
         const T f0 = h ? ((tq & 1) ? -n0 : n0) : T(1), df = h ? ((tq & 1) ? T(-2) : T(2)) : T(0);

@@ -752,11 +752,11 @@ constexpr int M64_COLS = 20, M64_PAD = 80, NBMAX64 = 8, SREC64 = RECW + 2;
 constexpr int SCF64 = NCM + 3;
 // nodes whose rows of the FP64 matrix a block holds: one chunk, or up to two
 // (more are read where they are)
-__host__ __device__ constexpr int m64_rows(bool one) { return one ? BASIS_NODES : 2 * BASIS_NODES; }
+__host__ __device__ constexpr int m64_rows(bool one, int S) { return one ? 8 * S : 2 * BASIS_NODES; }
 template <class T>
-__host__ __device__ constexpr size_t basis_table_bytes(bool one) {
+__host__ __device__ constexpr size_t basis_table_bytes(bool one, int S) {
     return sizeof(T) == 4 ? ((size_t)BASIS_NODES * (KM * 4 + 2) + (size_t)MMA_TABLE_FLOATS) * sizeof(float)
-                          : (size_t)m64_rows(one) * (M64_COLS + 2) * sizeof(T);
+                          : (size_t)m64_rows(one, S) * (M64_COLS + 2) * sizeof(T);
 }
 
 // Per warp: the own records of its 32/L bodies, then NBMAX neighbour
@@ -776,10 +776,10 @@ template <class T, int L>
 __host__ __device__ constexpr size_t walk_bytes_per_warp() {
     return FCC_WALK_SMEM ? (size_t)32 * slots_of(L) * 4 * sizeof(T) : 0;
 }
-template <class T, int L>
+template <class T, int L, int S>
 __host__ __device__ constexpr size_t stage_bytes_per_warp() {
     // FP64: 4 own and 4 x NBMAX64 neighbour records, the nodes' offsets and pressures, the own coefficients
-    if (sizeof(T) == 8) return (4 * (1 + NBMAX64) * SREC64 + 3 * 5 * 32 + 4 * SCF64) * sizeof(T);
+    if (sizeof(T) == 8) return (4 * (1 + NBMAX64) * SREC64 + 3 * S * 32 + 4 * SCF64) * sizeof(T);
     return (size_t)(32 / L) * (RECW + NBMAX * SRECW) * sizeof(T) + desc_slot_bytes<T>() + walk_bytes_per_warp<T, L>();
 }
 
@@ -1590,6 +1590,11 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
     constexpr bool MMA_S = MMA && FCC_MMA_SYNTH;
     constexpr int MPL = UpdatePre<T, L>::MPL;
     constexpr int SRW = SRECW;
+    // modes of the synthesis loop per pass: a LAT kernel, with a warp or two per
+    // SM, waits for instructions where the loop is unrolled (17% of its stalls;
+    // N = 1024 7.85 us a step unrolled, 7.60 by threes, 7.32 rolled); with 14
+    // warps the rolled loop's own instructions cost more (16384 22.4 / 22.8)
+    constexpr int MU = LAT ? 1 : KM;
     const int lane = threadIdx.x & 31;
     const int l = lane & (L - 1);
     const int g = wg * BPW + lane / L;
@@ -1797,7 +1802,7 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
             R2[sl] = T(0);
             if (v) vmask |= 1u << sl;
         }
-#pragma unroll
+#pragma unroll MU
         for (int m = 0; m < KM; ++m) {
             const T al = own[r_al(m)], be = own[r_be(m)];
             const T n = T(m + 2);
@@ -2227,7 +2232,7 @@ template <class T, int L, int S, bool ONE, int MODE, bool USER, bool LAT>
 __device__ __forceinline__ void forces_group(const DevPtrs<T>& d, int wg, T* stage, int par, const SimDesc<T>* sim0,
                                              const T* tab, int& cached, int* rbp, const BarrierLocal* lone,
                                              bool drawn, Resident<T, L>* res) {
-    if constexpr (sizeof(T) == 8) forces_warp64<ONE, MODE, USER, LAT>(d, wg, stage, par, sim0, tab, rbp, lone, drawn, res);
+    if constexpr (sizeof(T) == 8) forces_warp64<S, ONE, MODE, USER, LAT>(d, wg, stage, par, sim0, tab, rbp, lone, drawn, res);
     else forces_warp<T, L, S, ONE, MODE, USER, LAT>(d, wg, stage, par, sim0, tab, cached, rbp, lone, drawn, res);
 }
 
@@ -2458,28 +2463,28 @@ __device__ __forceinline__ const SimDesc<T>* copy_desc(const DevPtrs<T>& d) {
 
 // Dynamic shared memory of the force kernels: the FP32 mode table (one
 // contour chunk of nodes), then one neighbour stage per warp.
-template <class T, bool ONE>
+template <class T, bool ONE, int S>
 __device__ __forceinline__ T* warp_stage(size_t bytes_per_warp) {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
-    return reinterpret_cast<T*>(fcc_smem + basis_table_bytes<T>(ONE) + (threadIdx.x >> 5) * bytes_per_warp);
+    return reinterpret_cast<T*>(fcc_smem + basis_table_bytes<T>(ONE, S) + (threadIdx.x >> 5) * bytes_per_warp);
 }
 // the whole stage area of the block (every warp's stage, in order)
-template <class T, bool ONE>
+template <class T, bool ONE, int S>
 __device__ __forceinline__ unsigned char* block_stage_of() {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
-    return fcc_smem + basis_table_bytes<T>(ONE);
+    return fcc_smem + basis_table_bytes<T>(ONE, S);
 }
 
 // Copy the tables of a single-chunk kernel into shared memory: FP32 the mode
 // table of the first min(nth, BASIS_NODES) nodes and after it the tensor-core
 // fragment table, FP64 the contraction matrix and the nodes' (cos, sin).
 // Returns the table, or null when unused.
-template <class T, bool ONE>
+template <class T, bool ONE, int S>
 __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
     T* tab = reinterpret_cast<T*>(fcc_smem);
     if constexpr (sizeof(T) == 8) {  // M, then the nodes' (cos, sin)
-        constexpr int rows = m64_rows(ONE);
+        constexpr int rows = m64_rows(ONE, S);
         if (d.nth > rows) return nullptr;
         for (int u = threadIdx.x; u < rows * M64_COLS; u += blockDim.x) tab[u] = __ldg(d.basis + u);
         for (int u = threadIdx.x; u < 2 * d.nth; u += blockDim.x) tab[rows * M64_COLS + u] = __ldg(d.cs + u);
@@ -2508,7 +2513,7 @@ __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
 template <class T, int L, int S, bool ONE, bool SPLIT, int BLK, int MINB, bool USER = false>
 __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, int par0, LaunchStatus* status,
                                                     long long ticket) {
-    constexpr bool LAT = MINB == 1 && ONE && !SPLIT && L == 8 && S == 5;
+    constexpr bool LAT = MINB == 1 && ONE && !SPLIT && L == 8 && (S == 5 || sizeof(T) == 8);
     const int WPB = blockDim.x >> 5;  // at most BLK / 32
     const int warp = threadIdx.x >> 5;
     const int ngroups = (d.Ntot + (32 / L) - 1) / (32 / L);
@@ -2516,19 +2521,19 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
     const int g1 = (int)((long long)ngroups * (blockIdx.x + 1) / gridDim.x);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
-    T* stage = warp_stage<T, ONE>(stage_bytes_per_warp<T, L>());
-    const T* tab = stage_basis<T, ONE>(d);
+    T* stage = warp_stage<T, ONE, S>(stage_bytes_per_warp<T, L, S>());
+    const T* tab = stage_basis<T, ONE, S>(d);
     const SimDesc<T>* sim0 = copy_desc(d);
     __shared__ BarrierLocal bl;
     const bool lone = lone_sim(d);
     barrier_start(d.sync, bl, lone, d.flags, d.clock);
     int cached = -1;  // simulation whose descriptor this warp's slot holds
-    // FP32 with a single simulation: the warps of a block take its warp groups
-    // dynamically (measured: 1% faster at N = 16384).  Pools keep the static
-    // assignment (2% faster there: a warp that moves to another simulation's
-    // group re-copies the descriptor), and so does FP64 (one block of 8 warps
-    // per SM: 3% faster static).
-    const bool dyn = FCC_DYN && sizeof(T) == 4 && sim0 != nullptr;
+    // A single simulation: the warps of a block take its warp groups
+    // dynamically (measured: FP32 1% faster at N = 16384, FP64 in two blocks per
+    // SM 4% at 10000, 1% at 16384).  Pools keep the static assignment (2% faster
+    // there: a warp that moves to another simulation's group re-copies the
+    // descriptor), and so does FP64 in one block per SM (3% faster static).
+    const bool dyn = FCC_DYN && (sizeof(T) == 4 || MINB == 2) && sim0 != nullptr;
     __shared__ int s_next[2];  // next untaken warp group of the block, per step parity
     if (dyn && threadIdx.x == 0) s_next[0] = g0 + WPB;
     __syncthreads();
@@ -2546,8 +2551,8 @@ __global__ void __launch_bounds__(BLK, MINB) k_step(DevPtrs<T> d, int nsteps, in
         if (bl.any) {
             // the work list of a pool lives in the warps' stage area, free
             // between the closing barrier of a step and the forces
-            if (!rebuild_prologue(d, par, tid, nthr, bl, sim0, reinterpret_cast<int*>(block_stage_of<T, ONE>()),
-                                  (int)(WPB * stage_bytes_per_warp<T, L>() / sizeof(int))))
+            if (!rebuild_prologue(d, par, tid, nthr, bl, sim0, reinterpret_cast<int*>(block_stage_of<T, ONE, S>()),
+                                  (int)(WPB * stage_bytes_per_warp<T, L, S>() / sizeof(int))))
                 return;
             cached = -1;  // the descriptor slots were overwritten
             res.lists = false;
@@ -2657,8 +2662,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_gradients(DevPt
     const int wpb = blockDim.x >> 5;
     const int wg = blockIdx.x * wpb + (threadIdx.x >> 5);
     const int ngroups = (d.Ntot + (32 / L) - 1) / (32 / L);
-    T* stage = warp_stage<T, ONE>(stage_bytes_per_warp<T, L>());
-    const T* tab = stage_basis<T, ONE>(d);
+    T* stage = warp_stage<T, ONE, S>(stage_bytes_per_warp<T, L, S>());
+    const T* tab = stage_basis<T, ONE, S>(d);
     const SimDesc<T>* sim0 = copy_desc(d);
     int cached = -1;
     if (wg < ngroups)

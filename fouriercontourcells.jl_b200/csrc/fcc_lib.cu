@@ -214,6 +214,13 @@ void* step_fn(bool one, bool split) {
     return split ? (void*)k_step<T, L, S, false, true, BLK, MB> : (void*)k_step<T, L, S, false, false, BLK, MB>;
 }
 
+// a shape for contours of one chunk only
+template <class T, int L, int S, int BLK, int MB>
+void* step_fn_one(bool one, bool split) {
+    if (!one) return nullptr;
+    return split ? (void*)k_step<T, L, S, true, true, BLK, MB> : (void*)k_step<T, L, S, true, false, BLK, MB>;
+}
+
 // `family`: variants of one family give bit-identical trajectories (same
 // lanes x node slots, and — measured, since the compiler may fuse either
 // product of a*b + c*d differently under another register budget — the same
@@ -227,15 +234,16 @@ struct Variant {
 };
 
 const Variant VARIANTS[] = {
-    {8, 5, 256, 2, step_fn<float, 8, 5, 256, 2>, step_fn<double, 8, 5, 256, 1>, stage_bytes_per_warp<float, 8>(),
-     stage_bytes_per_warp<double, 8>(), 0},
-    {4, 10, 256, 2, step_fn<float, 4, 10, 256, 2>, nullptr, stage_bytes_per_warp<float, 4>(), 0, 1},
-    {16, 3, 256, 2, step_fn<float, 16, 3, 256, 2>, nullptr, stage_bytes_per_warp<float, 16>(), 0, 2},
-    {8, 5, 128, 5, step_fn<float, 8, 5, 128, 5>, nullptr, stage_bytes_per_warp<float, 8>(), 0, 3},
-    {16, 3, 128, 5, step_fn<float, 16, 3, 128, 5>, nullptr, stage_bytes_per_warp<float, 16>(), 0, 2},
-    {8, 5, 224, 2, step_fn<float, 8, 5, 224, 2>, step_fn<double, 8, 5, 224, 2>, stage_bytes_per_warp<float, 8>(),
-     stage_bytes_per_warp<double, 8>(), 0},
-    {8, 5, 256, 1, step_fn<float, 8, 5, 256, 1>, nullptr, stage_bytes_per_warp<float, 8>(), 0, 0},
+    {8, 5, 256, 2, step_fn<float, 8, 5, 256, 2>, step_fn<double, 8, 5, 256, 1>, stage_bytes_per_warp<float, 8, 5>(),
+     stage_bytes_per_warp<double, 8, 5>(), 0},
+    {4, 10, 256, 2, step_fn<float, 4, 10, 256, 2>, nullptr, stage_bytes_per_warp<float, 4, 10>(), 0, 1},
+    {16, 3, 256, 2, step_fn<float, 16, 3, 256, 2>, nullptr, stage_bytes_per_warp<float, 16, 3>(), 0, 2},
+    {8, 5, 128, 5, step_fn<float, 8, 5, 128, 5>, nullptr, stage_bytes_per_warp<float, 8, 5>(), 0, 3},
+    {16, 3, 128, 5, step_fn<float, 16, 3, 128, 5>, nullptr, stage_bytes_per_warp<float, 16, 3>(), 0, 2},
+    {8, 5, 224, 2, step_fn<float, 8, 5, 224, 2>, step_fn<double, 8, 5, 224, 2>, stage_bytes_per_warp<float, 8, 5>(),
+     stage_bytes_per_warp<double, 8, 5>(), 0},
+    {8, 5, 256, 1, step_fn<float, 8, 5, 256, 1>, nullptr, stage_bytes_per_warp<float, 8, 5>(), 0, 0},
+    {8, 8, 256, 1, nullptr, step_fn_one<double, 8, 8, 256, 1>, 0, stage_bytes_per_warp<double, 8, 8>(), 4},
 };
 constexpr int NVARIANTS = sizeof(VARIANTS) / sizeof(VARIANTS[0]);
 constexpr int LANES = 8, SLOTS = 5;  // compute_gradients and the FP64 step
@@ -885,10 +893,10 @@ struct Engine final : EngineBase {
     int variant = 0;
     const Variant& var() const { return VARIANTS[variant]; }
     static constexpr size_t grad_stage_bytes(bool one) {
-        return basis_table_bytes<T>(one) + (size_t)(256 / 32) * stage_bytes_per_warp<T, LANES>();
+        return basis_table_bytes<T>(one, SLOTS) + (size_t)(256 / 32) * stage_bytes_per_warp<T, LANES, SLOTS>();
     }
     size_t stage_bytes() const {
-        return basis_table_bytes<T>(nth <= var().L * var().S) + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
+        return basis_table_bytes<T>(nth <= var().L * var().S, var().S) + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
     }
     // compiled user terms: the 8 x 5 / 256-thread kernels with the user-term code
     bool user = false;
@@ -924,8 +932,10 @@ struct Engine final : EngineBase {
     //     224 wins where the 256-thread grid leaves its last round part-empty
     //     (N = 8280: 12.5 / 13.1 us; 16384: 22.7 / 23.1) and loses where both
     //     fill it (65536: 88.1 / 78.6).
-    // Contours of several chunks and parent drag keep the base shape: FP64
-    // variant 0, and 5 once a round of variant 0 does not hold the groups.
+    // Parent drag and contours of several chunks keep the base shape (FP64: 0
+    // or 5 as above), but for FP64 contours of 41 to 64 nodes in one round,
+    // which variant 7 takes in one chunk of 8 nodes a lane: 2304 bodies of 64
+    // nodes 14.4 us a step in two chunks, 11.6 in one.
     fcc_status choose_variant() {
         variant = 0;
         if (user) {  // one kernel family carries the user-term code
@@ -934,13 +944,16 @@ struct Engine final : EngineBase {
         }
         if (const char* e = std::getenv("FCC_VARIANT")) {
             const int v = std::atoi(e);
-            if (v >= 0 && v < NVARIANTS && (sizeof(T) == 4 || VARIANTS[v].f64)) variant = v;
+            if (v >= 0 && v < NVARIANTS && (sizeof(T) == 4 ? VARIANTS[v].f32 : VARIANTS[v].f64)) {
+                variant = v;
+                if (!step_kernel()) variant = 0;  // a shape that does not take this contour
+            }
             return FCC_OK;
         }
         if (N <= 0) return FCC_OK;
         const bool one_round = (N + 3) / 4 <= (int64_t)nsm * 8;
         if (sizeof(T) == 8) {
-            variant = one_round ? 0 : 5;
+            variant = !one_round ? 5 : nth > 40 && nth <= 64 ? 7 : 0;
             return FCC_OK;
         }
         if (!one_chunk() || split) return FCC_OK;

@@ -306,7 +306,7 @@ struct Pool final : PoolBase {
     bool split() const { return nsplit > 0; }
     void* step_kernel() const { return (sizeof(T) == 4 ? var().f32 : var().f64)(nth <= var().L * var().S, split()); }
     size_t stage_bytes() const {
-        return basis_table_bytes<T>(nth <= var().L * var().S) + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
+        return basis_table_bytes<T>(nth <= var().L * var().S, var().S) + (size_t)(var().blk / 32) * (sizeof(T) == 4 ? var().stage32 : var().stage64);
     }
 
     fcc_status init(const fcc_pool_params& q) {
@@ -614,8 +614,8 @@ struct Pool final : PoolBase {
 
     // ------------------------------------------------------------- run --
     fcc_status configure() {
-        if (variant >= 0 && sizeof(T) != 4 && !VARIANTS[variant].f64)
-            return fail(FCC_ERR_UNSUPPORTED, "pool: this kernel variant has no FP64 build");
+        if (variant >= 0 && (!(sizeof(T) == 4 ? VARIANTS[variant].f32 : VARIANTS[variant].f64) || !step_kernel()))
+            return fail(FCC_ERR_UNSUPPORTED, "pool: this kernel variant has no build for the pool's precision and contour");
         const int smem = (int)stage_bytes();
         CUDA_TRY(cudaFuncSetAttribute(step_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         int per_sm = 0;
@@ -945,9 +945,10 @@ struct Pool final : PoolBase {
         for (int pass = 0; pass < 2; ++pass)
         for (int v = 0; v < NVARIANTS; ++v) {
             const Variant& c = VARIANTS[v];
-            if (sizeof(T) != 4 && !c.f64) continue;
+            if (!(sizeof(T) == 4 ? c.f32 : c.f64)) continue;
             if (!reorder && c.family != cur.family) continue;
             variant = v;
+            if (!step_kernel()) continue;  // a shape that does not take this contour
             drop_graph();
             std::vector<long long> target(nslots, 0);
             for (int s : order) target[s] = slots[s].clock_h + steps;
@@ -1096,8 +1097,8 @@ struct Pool final : PoolBase {
 
     fcc_status config(int32_t v, int32_t steps) override {
         if (v < -1 || v >= NVARIANTS) return fail(FCC_ERR_ARGUMENT, "pool: no such kernel variant");
-        if (v >= 0 && sizeof(T) != 4 && !VARIANTS[v].f64)
-            return fail(FCC_ERR_UNSUPPORTED, "pool: this kernel variant has no FP64 build");
+        if (v >= 0 && !(sizeof(T) == 4 ? VARIANTS[v].f32 : VARIANTS[v].f64))
+            return fail(FCC_ERR_UNSUPPORTED, "pool: this kernel variant has no build of the pool's precision");
         if (steps < 0) return fail(FCC_ERR_ARGUMENT, "pool: steps per launch must be >= 0");
         variant = v;
         user_set = v >= 0;

@@ -120,3 +120,28 @@ def test_one_round_shapes_give_the_bits_of_the_others(n, monkeypatch):
         assert nb == builds
         for f in ("x", "y", "θ", "coef", "imgx", "imgy"):
             assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
+@pytest.mark.parametrize("nθ,n", [(41, 61), (48, 62), (57, 64), (64, 30)])
+def test_fp64_shapes_of_finer_contours_give_the_same_bits(nθ, n, monkeypatch):
+    """Contours of 41 to 64 nodes in one chunk of 8 nodes a lane (the choice for
+    one round of warp groups) against two chunks, and in a pool: a simulation's
+    result does not depend on the shape its size, or its pool's, selects."""
+    bodies, box = deformed(8, 8, 10, n)
+    bodies = take(bodies, n)
+    out = []
+    for v in (None, "0", "5", "7"):
+        if v is None:
+            monkeypatch.delenv("FCC_VARIANT", raising=False)
+        else:
+            monkeypatch.setenv("FCC_VARIANT", v)
+        s = fcc.Simulation(bodies, box, T=np.float64, nθ=nθ, **KW)
+        s.run(60)
+        out.append(s.bodies)
+    pool = fcc.Pool(T=np.float64, nθ=nθ, max_bodies=256, max_cells=256, max_sims=2)
+    slot = pool.add(bodies, box, horizon=60, **KW)
+    pool.run(60)
+    out.append(pool.bodies(slot))
+    for b in out[1:]:
+        for f in ("x", "y", "θ", "coef"):
+            assert np.array_equal(getattr(out[0], f), getattr(b, f)), f
