@@ -2456,7 +2456,8 @@ __device__ __forceinline__ const SimDesc<T>* copy_desc(const DevPtrs<T>& d) {
     __shared__ __align__(16) unsigned s_desc[(sizeof(SimDesc<T>) + 3) / 4];
     if (d.nsims != 1) return nullptr;
     const unsigned* src = reinterpret_cast<const unsigned*>(d.sims);
-    for (int u = threadIdx.x; u < (int)((sizeof(SimDesc<T>) + 3) / 4); u += blockDim.x) s_desc[u] = src[u];
+    for (int u = threadIdx.x; u < (int)(sizeof(SimDesc<T>) / 4); u += blockDim.x) cp_async4(s_desc + u, src + u);
+    cp_async_wait_all();
     __syncthreads();
     return reinterpret_cast<const SimDesc<T>*>(s_desc);
 }
@@ -2483,25 +2484,33 @@ template <class T, bool ONE, int S>
 __device__ __forceinline__ const T* stage_basis(const DevPtrs<T>& d) {
     extern __shared__ __align__(16) unsigned char fcc_smem[];
     T* tab = reinterpret_cast<T*>(fcc_smem);
+    // asynchronous copies, all in flight at once: with one warp per block the
+    // loads of a loop cost a launch 4 us
+    auto copy = [&](void* to, const void* from, int bytes) {  // multiples of 16 bytes, or of 8
+        if (bytes & 15) {
+            for (int u = 8 * threadIdx.x; u < bytes; u += 8 * blockDim.x)
+                cp_async8(static_cast<char*>(to) + u, static_cast<const char*>(from) + u);
+        } else {
+            for (int u = 16 * threadIdx.x; u < bytes; u += 16 * blockDim.x)
+                cp_async16(static_cast<char*>(to) + u, static_cast<const char*>(from) + u);
+        }
+    };
     if constexpr (sizeof(T) == 8) {  // M, then the nodes' (cos, sin)
         constexpr int rows = m64_rows(ONE, S);
         if (d.nth > rows) return nullptr;
-        for (int u = threadIdx.x; u < rows * M64_COLS; u += blockDim.x) tab[u] = __ldg(d.basis + u);
-        for (int u = threadIdx.x; u < 2 * d.nth; u += blockDim.x) tab[rows * M64_COLS + u] = __ldg(d.cs + u);
-        __syncthreads();
-        return tab;
+        copy(tab, d.basis, rows * M64_COLS * 8);
+        copy(tab + rows * M64_COLS, d.cs, 16 * d.nth);
+    } else {
+        if (!ONE) return nullptr;
+        // the mode table, the tensor-core fragments and the nodes' (cos, sin): an
+        // acquire at a grid barrier empties L1, so read from global memory the
+        // last cost a trip to L2 every step
+        const int n = min(d.nth, BASIS_NODES);
+        copy(tab, d.basis, n * KM * 16);
+        if (d.mtab) copy(tab + BASIS_NODES * KM * 4, d.mtab, MMA_TABLE_FLOATS * 4);
+        copy(tab + BASIS_NODES * KM * 4 + MMA_TABLE_FLOATS, d.cs, 8 * n);
     }
-    if (!ONE) return nullptr;
-    const int n = min(d.nth, BASIS_NODES) * KM * 4;
-    for (int u = threadIdx.x; u < n; u += blockDim.x) tab[u] = __ldg(d.basis + u);
-    if (d.mtab) {  // the tensor-core fragments follow the mode table
-        float* mt = reinterpret_cast<float*>(fcc_smem) + BASIS_NODES * KM * 4;
-        for (int u = threadIdx.x; u < MMA_TABLE_FLOATS; u += blockDim.x) mt[u] = __ldg(d.mtab + u);
-    }
-    // and the nodes' (cos, sin): an acquire at a grid barrier empties L1, so
-    // read from global memory they cost a trip to L2 every step
-    for (int u = threadIdx.x; u < 2 * min(d.nth, BASIS_NODES); u += blockDim.x)
-        tab[BASIS_NODES * KM * 4 + MMA_TABLE_FLOATS + u] = __ldg(d.cs + u);
+    cp_async_wait_all();
     __syncthreads();
     return tab;
 }
