@@ -56,27 +56,6 @@ __device__ __forceinline__ void load_head(const double* p, double& x, double& y,
     double2 b = ldcg(reinterpret_cast<const double2*>(p) + 1);
     x = a.x, y = a.y, rm = b.x, w = b.y;
 }
-// R0-scaled lab coefficients of a record (slots 4..22; slot 23 comes along)
-__device__ __forceinline__ void load_lab(const float* p, float (&c)[20]) {
-    const float4* q = reinterpret_cast<const float4*>(p + R_A0);
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-        float4 v = ldcg(q + u);
-        c[4 * u] = v.x;
-        c[4 * u + 1] = v.y;
-        c[4 * u + 2] = v.z;
-        c[4 * u + 3] = v.w;
-    }
-}
-__device__ __forceinline__ void load_lab(const double* p, double (&c)[20]) {
-    const double2* q = reinterpret_cast<const double2*>(p + R_A0);
-#pragma unroll
-    for (int u = 0; u < 10; ++u) {
-        double2 v = ldcg(q + u);
-        c[2 * u] = v.x;
-        c[2 * u + 1] = v.y;
-    }
-}
 
 // The current record buffer is rec[par], par = parity of the engine's step
 // counter (all simulations of an engine advance together; a frozen one
@@ -108,27 +87,9 @@ __device__ __forceinline__ float4 lds4(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 #endif
 }
-struct Double4 {
-    double x, y, z, w;
-};
-__device__ __forceinline__ Double4 lds4(const double* p) { return Double4{p[0], p[1], p[2], p[3]}; }
 __device__ __forceinline__ void lds_head(const float* p, float& x, float& y, float& rm, float& w) {
     const float4 v = lds4(p);
     x = v.x, y = v.y, rm = v.z, w = v.w;
-}
-__device__ __forceinline__ void lds_head(const double* p, double& x, double& y, double& rm, double& w) {
-    x = p[R_X], y = p[R_Y], rm = p[R_RMAX], w = p[R_W];
-}
-__device__ __forceinline__ void lds_lab(const float* p, float (&c)[20]) {
-#pragma unroll
-    for (int u = 0; u < 5; ++u) {
-        const float4 v = lds4(p + R_A0 + 4 * u);
-        c[4 * u] = v.x, c[4 * u + 1] = v.y, c[4 * u + 2] = v.z, c[4 * u + 3] = v.w;
-    }
-}
-__device__ __forceinline__ void lds_lab(const double* p, double (&c)[20]) {
-#pragma unroll
-    for (int u = 0; u < 20; ++u) c[u] = p[R_A0 + u];
 }
 
 // R_j(psi) = R0 [a0 + sum_n alpha_n cos n psi + beta_n sin n psi] of a staged
@@ -210,26 +171,11 @@ __device__ __forceinline__ float radius_at(const float* p, float cp, float sp) {
     return a0 + (re + ro);
 #endif
 }
-__device__ __forceinline__ double radius_at(const double* p, double cp, double sp) {
-    double c = cp, sn = sp, r = p[R_A0];
-#pragma unroll
-    for (int m = 0; m < KM; ++m) {
-        const double cn = c * cp - sn * sp;
-        sn = sn * cp + c * sp;
-        c = cn;
-        r += p[r_al(m)] * c + p[r_be(m)] * sn;
-    }
-    return r;
-}
 
 // |u| and 1/|u| of a contour node distance (FP32: one rsqrt)
 __device__ __forceinline__ void norm_inv(float x2, float& n, float& inv) {
     inv = rsqrtf(x2);
     n = x2 * inv;
-}
-__device__ __forceinline__ void norm_inv(double x2, double& n, double& inv) {
-    n = sqrt(x2);
-    inv = 1.0 / n;
 }
 
 __device__ __forceinline__ int jmod(int a, int n) {
@@ -725,7 +671,7 @@ constexpr int NBMAX = 12;
 constexpr int SRECW = RECW + 4;
 
 #ifndef FCC_DYN
-#define FCC_DYN 1  // 1: FP32, one simulation: warps take their block's warp groups dynamically
+#define FCC_DYN 1  // 1: one simulation, two blocks per SM: warps take their block's warp groups dynamically
 #endif
 
 // FP32 single-chunk kernels read cos(n phi_k), sin(n phi_k) (and n times
@@ -813,7 +759,7 @@ __host__ __device__ constexpr int draw_ahead_slot() {
 // pairs, rows of 8 floats with the columns of rows 4..7 (mod 8) rotated by 4
 // words: conflict-free both ways.
 #ifndef FCC_MMA_SYNTH
-#define FCC_MMA_SYNTH 0  // 1: contour synthesis on the tensor cores too (measured: slower, see DESIGN)
+#define FCC_MMA_SYNTH 0  // 1: contour synthesis on the tensor cores too (measured: slower: the derivative's coefficients are staged and it spills)
 #endif
 
 __device__ __forceinline__ uint32_t tf32_rna(float x) {
@@ -1851,17 +1797,21 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         for (int u = 0; u < MUT; ++u) {
 #pragma unroll
             for (int j = 0; j < fcc_user::MAX_M; ++j) UQ[u][j] = T(0);
-            if (u >= P.nub || !((P.ub_mask[u] >> ti) & 1u)) continue;
+            if (u < P.nub && ((P.ub_mask[u] >> ti) & 1u)) {
 #pragma unroll
-            for (int sl = 0; sl < S; ++sl)
-                if (vmask & (1u << sl)) {
-                    T q[fcc_user::MAX_M] = {};
-                    fcc_user::body_q<T>(P.ub_id[u], R[sl], R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], q);
+                for (int sl = 0; sl < S; ++sl)
+                    if (vmask & (1u << sl)) {
+                        T q[fcc_user::MAX_M] = {};
+                        fcc_user::body_q<T>(P.ub_id[u], R[sl], R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], q);
 #pragma unroll
-                    for (int j = 0; j < fcc_user::MAX_M; ++j) UQ[u][j] += q[j];
-                }
+                        for (int j = 0; j < fcc_user::MAX_M; ++j) UQ[u][j] += q[j];
+                    }
+            }
+            // every lane of the warp takes the shuffles: it may hold bodies of several types
+            if (u < P.nub) {
 #pragma unroll
-            for (int j = 0; j < fcc_user::MAX_M; ++j) UQ[u][j] = group_sum<L>(UQ[u][j]) * dphi;
+                for (int j = 0; j < fcc_user::MAX_M; ++j) UQ[u][j] = group_sum<L>(UQ[u][j]) * dphi;
+            }
         }
     }
 

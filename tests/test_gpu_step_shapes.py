@@ -145,3 +145,23 @@ def test_fp64_shapes_of_finer_contours_give_the_same_bits(nθ, n, monkeypatch):
     for b in out[1:]:
         for f in ("x", "y", "θ", "coef"):
             assert np.array_equal(getattr(out[0], f), getattr(b, f)), f
+
+
+def test_user_body_terms_on_alternating_types():
+    """User terms restricted to one type each, the types alternating within a
+    warp's bodies: forces of both precisions against the FP64 oracle (FP64 at
+    1e-12 of each field's scale, FP32 at 1e-5 on an FP32-representable state, as
+    the other user-term tests; no contacts, so no Heaviside flips)."""
+    bodies, box = deformed(6, 6, 6, 17, packing=0.6)
+    bodies.type[:] = 1 + np.arange(bodies.n) % 2
+    for f in ("x", "y", "θ", "coef", "R0"):
+        getattr(bodies, f)[...] = np.asarray(getattr(bodies, f), np.float32)
+    kw = {**KW, "energies": (fcc.Tension(0.02), fcc.OnTypes(fcc.ShapeIndexElasticity(0.05, 3.7), 1),
+                             fcc.OnTypes(fcc.Bending(0.02), 2))}
+    o = oracle.OracleSimulation(bodies, box, T=np.float64, **kw).refresh()
+    for T, tol in ((np.float64, 1e-12), (np.float32, 1e-5)):
+        g = fcc.Simulation(bodies, box, T=T, **kw).refresh()
+        for f in ("GR", "GD", "GDD", "glab", "gcoef", "Ebody"):
+            assert relerr(getattr(g.grad, f), getattr(o.grad, f)) < tol, (T, f)
+        g.run(3)
+        assert np.isfinite(g.bodies.coef).all()
