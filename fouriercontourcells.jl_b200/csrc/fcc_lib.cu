@@ -686,6 +686,7 @@ struct Engine final : EngineBase {
     double last_ms = 0;
     int64_t last_launches = 0, last_steps = 0;
     int step_grid = 0, step_blk = 0;  // launch shape of the step kernel
+    int rebuild_grid = 0;             // blocks of k_rebuild
     // device buffers
     DBuf<SimDesc<T>> sims;
     DBuf<T> rec0, rec1, coef, R0, x0, y0, rmax0, cs, basis, gx, gy, gth, glab, E, P, GR, GD, GDD, gcoef;
@@ -1082,6 +1083,15 @@ struct Engine final : EngineBase {
         return FCC_OK;
     }
 
+    // Wait for the launches queued and take the status the last one left.
+    fcc_status launch_status(LaunchStatus& ls) {
+        FCC_TRY(sync_stream());
+        std::memcpy(&ls, ls_h, sizeof(ls));  // written by the device before the stream was done
+        if (ls.ticket != ticket || ls.error)
+            return fail(FCC_ERR_DEVICE, "a grid barrier wait timed out in the step kernel");
+        return FCC_OK;
+    }
+
     // Account executed steps (t accumulates in T, as sim.t += sim.dt does).
     void account(long long newclock) {
         const long long executed = newclock - clock_h;
@@ -1131,11 +1141,8 @@ struct Engine final : EngineBase {
             }
             // the kernel itself leaves its status for the host: no copy, one synchronisation
             CUDA_TRY(cudaEventRecord(ev1, stream));
-            FCC_TRY(sync_stream());
             LaunchStatus ls;
-            std::memcpy(&ls, ls_h, sizeof(ls));  // written by the device before the stream was done
-            if (ls.ticket != ticket || ls.error)
-                return fail(FCC_ERR_DEVICE, "a grid barrier wait timed out in the step kernel");
+            FCC_TRY(launch_status(ls));
             account(ls.clock);
             const int64_t executed = ls.clock - start;
             done += executed;
@@ -1186,27 +1193,31 @@ struct Engine final : EngineBase {
     fcc_status update_neighbors(bool force) override {
         Range range("fcc update_neighbors");
         if (!has_contact || N == 0) return FCC_OK;
-        const DevPtrs<T> d = ptrs();
-        const int grid = (int)((N + 255) / 256);
+        if (!rebuild_grid) {
+            int per_sm = 0;
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rebuild<T>, REBUILD_BLOCK, 0));
+            if (per_sm < 1) return fail(FCC_ERR_UNSUPPORTED, "rebuild kernel does not fit on an SM");
+            rebuild_grid = (int)std::min<int64_t>(neighbor_grid(N), (int64_t)per_sm * nsm);
+        }
         for (int attempt = 0; attempt < 8; ++attempt) {
-            DevPtrs<T> dd = ptrs();
+            DevPtrs<T> d = ptrs();
+            int p0 = par();
             if (!force && attempt == 0) {
-                k_skin_check<T><<<grid, 256, 0, stream>>>(dd, par());
+                k_skin_check<T><<<(int)((N + 255) / 256), 256, 0, stream>>>(d, p0);
                 CUDA_TRY(cudaGetLastError());
             }
-            k_prepare_rebuild<T><<<1, 256, 0, stream>>>(dd, (force || attempt > 0) ? 1 : 0);
-            k_phase_count<T><<<grid, 256, 0, stream>>>(dd, par());
-            k_phase_scan<T><<<scan_grid(ncx * ncy), 256, 0, stream>>>(dd);
-            k_phase_scatter<T><<<grid, 256, 0, stream>>>(dd);
-            k_phase_sort<T><<<(ncx * ncy + 255) / 256, 256, 0, stream>>>(dd);
-            k_phase_neighbors<T><<<neighbor_grid(N), 256, 0, stream>>>(dd, par());
-            k_finish_rebuild<T><<<1, 256, 0, stream>>>(dd);
+            k_prepare_rebuild<T><<<1, 256, 0, stream>>>(d, (force || attempt > 0) ? 1 : 0);
             CUDA_TRY(cudaGetLastError());
+            ++ticket;
+            void* args[] = {&d, &p0, &ls_d, &ticket};
+            CUDA_TRY(cudaLaunchCooperativeKernel((void*)k_rebuild<T>, dim3(rebuild_grid), dim3(REBUILD_BLOCK), args, 0,
+                                                 stream));
+            LaunchStatus ls;
+            FCC_TRY(launch_status(ls));
+            if (!(ls.flags & F_FROZEN)) return FCC_OK;
             FCC_TRY(read_status());
-            if (!(st_h->flags & F_FROZEN)) return FCC_OK;
             FCC_TRY(regrow());
         }
-        (void)d;
         return fail(FCC_ERR_DEVICE, "neighbour list did not fit after regrowth");
     }
 

@@ -165,3 +165,36 @@ def test_user_body_terms_on_alternating_types():
             assert relerr(getattr(g.grad, f), getattr(o.grad, f)) < tol, (T, f)
         g.run(3)
         assert np.isfinite(g.bodies.coef).all()
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("nx,ny,n,cap", [(8, 8, 1, None), (8, 8, 33, 1), (18, 16, 257, None), (150, 140, 20999, 4)])
+def test_update_neighbors_lists_and_flags(nx, ny, n, cap, T):
+    """The stand-alone rebuild over its grids (one block, a remainder, more
+    bodies than the grid's lanes) and with lists that have to grow: the
+    oracle's lists (FP64; integers: equality), a rebuild only where one is due,
+    and steps that go on from it as from the rebuild of a first step."""
+    bodies, box = deformed(nx, ny, 6, 23)
+    bodies = take(bodies, n)
+    kw = {**KW, "T": T, **({} if cap is None else {"nl_capacity": cap})}
+    g = fcc.Simulation(bodies, box, **kw)
+    g.update_neighbors()
+    a = g.neighbors
+    if cap is not None:
+        assert a.cap >= a.count.max() > cap
+    if T is np.float64:
+        o = oracle.OracleSimulation(bodies, box, **{**KW, "T": T})
+        o.update_neighbors()
+        b = o.neighbors
+        for f in ("cellid", "perm", "start", "stop", "count"):
+            assert np.array_equal(getattr(a, f), getattr(b, f)), f
+        listed = np.arange(min(a.idx.shape[0], b.idx.shape[0]))[:, None] < a.count
+        assert np.array_equal(a.idx[:len(listed)][listed], b.idx[:len(listed)][listed])
+    builds = g.builds
+    assert g.update_neighbors().builds == builds
+    assert g.update_neighbors(force=True).builds == builds + 1
+    fresh = fcc.Simulation(bodies, box, **kw)
+    g.run(5)
+    fresh.run(5)
+    for f in ("x", "y", "θ", "coef"):
+        assert np.array_equal(getattr(g.bodies, f), getattr(fresh.bodies, f)), f
