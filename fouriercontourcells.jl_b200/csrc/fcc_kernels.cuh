@@ -2630,8 +2630,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_gradients(DevPt
                                                            nullptr);
 }
 
-// Stand-alone rebuild phases (update_neighbors!, and the stateless neighbour
-// build), one launch per phase.
+// Phases of the stateless neighbour builds, one launch per phase.
 template <class T>
 __global__ void k_phase_count(DevPtrs<T> d, int par) {
     if (ldcg(&d.sync->any_need))
