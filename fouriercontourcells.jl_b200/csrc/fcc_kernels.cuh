@@ -1355,16 +1355,20 @@ struct UserBody {
             T dq[fcc_user::MAX_M][3] = {};                                                                   \
             fcc_user::F::dq(v ? R[sl] : T(1), R1[sl], R2[sl], P.ub_a[u], P.ub_b[u], dq);                     \
             _Pragma("unroll") for (int j = 0; j < fcc_user::MAX_M; ++j) {                                    \
-                const T wj = v ? w[u][j] : T(0);                                                             \
-                GR[sl] += wj * dq[j][0];                                                                     \
-                GD[sl] += wj * dq[j][1];                                                                     \
-                GDD[sl] += wj * dq[j][2];                                                                    \
+                GR[sl] += w[u][j] * dq[j][0];                                                                \
+                GD[sl] += w[u][j] * dq[j][1];                                                                \
+                GDD[sl] += w[u][j] * dq[j][2];                                                               \
             }                                                                                                \
         }                                                                                                    \
     }
             FCC_USER_BODY_TERMS(FCC_UT_CASE)
 #undef FCC_UT_CASE
         }
+        // a node beyond the contour has no gradients: what the terms gave there
+        // (infinite or NaN for some) is dropped, as a zero weight would not
+#pragma unroll
+        for (int sl = 0; sl < S; ++sl)
+            if (!(vmask & (1u << sl))) GR[sl] = GD[sl] = GDD[sl] = T(0);
     }
 };
 

@@ -25,6 +25,8 @@
  *   dq(R, dR, ddR, a, b, out[M][3])                 dq_j / d(R, R', R'')
  *   F (Q[M], R0, type, a, b) -> E                   energy of the integrals
  *   dF(Q[M], R0, type, a, b, out[M])                dF / dQ_j
+ *   (q and dq may also be called off the contour, at R = 1, R' = R'' = 0;
+ *   what they return there is dropped, whatever it is)
  * Contact terms:
  *   g(d, ti, tj, related, a, b) -> energy density at penetration depth d
  *                                  (d > 0 inside the neighbour; types 1-based)

@@ -1,0 +1,55 @@
+"""Device helpers on their own (marked ``gpu``): device_units.cu, compiled with
+the library's flags, calls them at the arguments that whole simulations reach
+rarely or not at all."""
+
+import ctypes as C
+import os
+import re
+import shlex
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import PKG_DIR
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def unit(tmp_path_factory):
+    """unit(name, *arguments): arrays go as pointers, the returned CUDA error
+    must be 0."""
+    make = open(os.path.join(PKG_DIR, "csrc", "Makefile")).read().replace("\\\n", " ")
+    flags = re.search(r"^NVFLAGS\s*:=(.*)$", make, re.M)[1]
+    flags = [f for f in shlex.split(flags.replace("$(HOSTCXX)", "g++")) if f not in ("-Xptxas", "-v")]
+    so = str(tmp_path_factory.mktemp("units") / "units.so")
+    nvcc = "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc if os.path.exists(nvcc) else "nvcc", *flags, "-shared", "-o", so,
+                    os.path.join(HERE, "device_units.cu")], check=True)
+    lib = C.CDLL(so)
+
+    def call(name, *args):
+        c = {int: C.c_int, float: C.c_double}
+        got = getattr(lib, name)(*(c[type(a)](a) if type(a) in c else C.c_void_p(a.ctypes.data) for a in args))
+        assert got == 0, (name, got)
+    return call
+
+
+@pytest.mark.parametrize("nθ", [5, 24, 37, 40])
+def test_user_term_that_is_singular_on_a_circle(unit, nθ):
+    """A term whose derivative does not exist where R' = R'' = 0, on deformed
+    contours: the slots beyond a contour add nothing, the others w dq (the same
+    IEEE operations in numpy; R' / s to one rounding of each: 4 ulp)."""
+    rng = np.random.default_rng(nθ)
+    R, R1, R2 = (v + rng.standard_normal((32, 5)) * 0.2 for v in (1.0, 0.0, 0.0))
+    out = [np.zeros((32, 5)) for _ in range(3)]
+    w = 0.7
+    unit("unit_user_gradients", nθ, R, R1, R2, w, *out)
+    node = np.arange(32)[:, None] % 8 + 8 * np.arange(5)
+    s = np.sqrt(R1 ** 2 + R2 ** 2)
+    for got, want in zip(out, (0 * R, w * R1 / s, w * R2 / s)):
+        assert np.array_equal(got[node >= nθ], np.zeros((node >= nθ).sum()))
+        assert np.allclose(got[node < nθ], want[node < nθ], rtol=4 * 2.0 ** -52, atol=0)
