@@ -439,8 +439,12 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
 #pragma unroll
         for (int sl = 0; sl < S; ++sl) {  // nodes beyond the contour: no branch, their value is dropped
             const bool v = vmask & (1u << sl);
-            const T x2 = v ? R[sl] * R[sl] + R1[sl] * R1[sl] : T(1);
-            const T q = x2 * rsqrt_normal(x2);
+            // the smallest normal number is lost in any sum but at R = R' = 0 (a
+            // shape at its bound may touch the centre), where the root of 0 is 0
+            // to 1e-154 instead of 0 times infinity; it costs no instruction (a
+            // comparison a node: 884 against 904 us a pass of 1024 bodies)
+            const T x2 = fma(R[sl], R[sl], fma(R1[sl], R1[sl], T(2.2250738585072014e-308)));
+            const T q = x2 * rsqrt_normal(v ? x2 : T(1));
             Qp += v ? q : T(0);
         }
     }

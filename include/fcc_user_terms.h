@@ -49,6 +49,7 @@
 #if defined(__CUDACC__)
 namespace fcc {
 __device__ __forceinline__ double rsqrt_normal(double x);
+__device__ __forceinline__ double sqrt_normal(double x);
 }
 #endif
 
@@ -61,6 +62,15 @@ FCC_HD double inv_sqrt(double x) {
     return fcc::rsqrt_normal(x);
 #else
     return 1.0 / sqrt(x);
+#endif
+}
+
+/* sqrt(x) for x >= 0 in FP64 likewise. */
+FCC_HD double root(double x) {
+#if defined(__CUDA_ARCH__)
+    return fcc::sqrt_normal(x);
+#else
+    return sqrt(x);
 #endif
 }
 
@@ -109,7 +119,7 @@ struct ShapeIndexElasticity {
     static constexpr int M = 2;
     template <class T>
     FCC_HD static void q(T R, T dR, T, T, T, T* out) {
-        if constexpr (sizeof(T) == 8) out[0] = (R * R + dR * dR) * inv_sqrt(R * R + dR * dR);
+        if constexpr (sizeof(T) == 8) out[0] = root(R * R + dR * dR);
         else out[0] = sqrt(R * R + dR * dR);
         out[1] = R * R / T(2);
     }
