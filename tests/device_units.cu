@@ -72,7 +72,22 @@ __global__ void k_user_gradients(SimDesc<double>* P, int nth, const double* R, c
     u.gradients(*P, 0, vmask, r, r1, r2, gr, gd, gdd);
     for (int s = 0; s < 5; ++s) GR[5 * t + s] = gr[s], GD[5 * t + s] = gd[s], GDD[5 * t + s] = gdd[s];
 }
+__global__ void k_roots(const double* x, int n, double* inv, double* root) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    inv[i] = rsqrt_normal(x[i]);
+    root[i] = sqrt_normal(x[i]);
+}
 }  // namespace
+
+extern "C" int unit_roots(const double* x, int n, double* inv, double* root) {
+    Dev<double> dx(x, n), di(inv, n), dr(root, n);
+    for (cudaError_t e : {dx.e, di.e, dr.e}) TRY(e);
+    k_roots<<<(n + 255) / 256, 256>>>(dx.p, n, di.p, dr.p);
+    TRY(cudaGetLastError());
+    TRY(di.back(inv));
+    return (int)dr.back(root);
+}
 
 extern "C" int unit_user_gradients(int nth, const double* R, const double* R1, const double* R2, double w, double* GR,
                                    double* GD, double* GDD) {

@@ -53,3 +53,29 @@ def test_user_term_that_is_singular_on_a_circle(unit, nθ):
     for got, want in zip(out, (0 * R, w * R1 / s, w * R2 / s)):
         assert np.array_equal(got[node >= nθ], np.zeros((node >= nθ).sum()))
         assert np.allclose(got[node < nθ], want[node < nθ], rtol=4 * 2.0 ** -52, atol=0)
+
+
+def test_fp64_roots_over_the_exponents(unit):
+    """rsqrt_normal and sqrt_normal against 80-bit roots.  Bounds in units in
+    the last place: the final rounding (1/2), for the reciprocal the rounding of
+    x y in the residual (half of 2^-53, at most 1/2 ulp) and the cubic's
+    remainder (5/16 (2^-19)^3, 0.02 ulp), for the root the rounding of a residual
+    that is subnormal for the smallest x (1/4): 1.1 and 1."""
+    rng = np.random.default_rng(1)
+    tiny, huge = np.finfo(np.float64).tiny, np.finfo(np.float64).max
+    edge = np.ldexp(1.0, np.arange(-1021, 1024))
+    x = np.concatenate([np.ldexp(1 + rng.random(400_000), rng.integers(-1022, 1024, 400_000)),
+                        np.nextafter(edge, 0), edge, np.nextafter(edge, np.inf), 1 + rng.random(100_000) * 3,
+                        [tiny, huge]])
+    inv, root = np.zeros_like(x), np.zeros_like(x)
+    unit("unit_roots", x, len(x), inv, root)
+    exact = np.sqrt(x.astype(np.longdouble))
+    for got, want, bound in ((inv, 1 / exact, 1.1), (root, exact, 1.0)):
+        ulp = np.spacing(want.astype(np.float64)).astype(np.longdouble)
+        assert (np.abs(got - want) / ulp).max() <= bound
+    x = np.array([0.0, 5e-324, 1e-320, 1e-310, np.nextafter(tiny, 0), np.inf, np.nan])
+    inv, root = np.zeros_like(x), np.zeros_like(x)
+    unit("unit_roots", x, len(x), inv, root)
+    assert root[0] == 0 and root[5] == np.inf and np.isnan(root[6])
+    # below the smallest normal number: within that number's root of the value
+    assert (np.abs(root[1:5] - np.sqrt(x[1:5])) <= np.sqrt(tiny)).all()
