@@ -860,13 +860,10 @@ struct Pool final : PoolBase {
         if (user_set) return FCC_OK;
         std::lock_guard<std::mutex> lk(tune_mutex());
         auto it = tune_table().find(bucket());
-        if (it != tune_table().end()) {
-            variant = it->second;
-            tuned = true;
-        } else {
-            variant = -1;
-            tuned = false;
-        }
+        variant = it != tune_table().end() ? it->second : -1;
+        // tuned on another contour, by a shape that does not take this one's nodes
+        if (variant >= 0 && !step_kernel()) variant = -1;
+        tuned = variant >= 0;
         return FCC_OK;
     }
 

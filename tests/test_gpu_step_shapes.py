@@ -198,3 +198,23 @@ def test_update_neighbors_lists_and_flags(nx, ny, n, cap, T):
     fresh.run(5)
     for f in ("x", "y", "θ", "coef"):
         assert np.array_equal(getattr(g.bodies, f), getattr(fresh.bodies, f)), f
+
+
+def test_a_tuned_shape_does_not_bind_other_contours():
+    """The tuner remembers a launch shape by size and precision; a pool of that
+    size whose contour the shape does not take (here 80 nodes, after one of 64
+    was tuned, where the shape of one chunk of 8 nodes a lane is the fastest)
+    runs with its own and equals the simulation alone."""
+    bodies, box = deformed(8, 8, 10, 5)
+    tuned = fcc.Pool(T=np.float64, nθ=64, max_bodies=256, max_cells=256, max_sims=2)
+    tuned.add(bodies, box, horizon=1 << 20, **KW)
+    tuned.run(5)
+    tuned.tune(steps=40, reorder=True)
+    pool = fcc.Pool(T=np.float64, nθ=80, max_bodies=256, max_cells=256, max_sims=2)
+    slot = pool.add(bodies, box, horizon=60, **KW)
+    pool.run(60)
+    alone = fcc.Simulation(bodies, box, T=np.float64, nθ=80, **KW)
+    alone.run(60)
+    a, b = alone.bodies, pool.bodies(slot)
+    for f in ("x", "y", "θ", "coef"):
+        assert np.array_equal(getattr(a, f), getattr(b, f)), f
