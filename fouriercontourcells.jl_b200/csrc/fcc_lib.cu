@@ -61,6 +61,7 @@ fcc_status fail(fcc_status code, const std::string& msg) {
 }
 fcc_status cuda_fail(cudaError_t e, const char* what) {
     g_err = std::string(what) + ": " + cudaGetErrorString(e);
+    (void)cudaGetLastError();  // reported here: the check after the next launch must not find it again
     return e == cudaErrorMemoryAllocation ? FCC_ERR_NOMEM : FCC_ERR_CUDA;
 }
 #define CUDA_TRY(x)                                      \
@@ -1801,8 +1802,8 @@ fcc_status fcc_host_alloc(int64_t bytes, void** out) {
     if (bytes == 0) return FCC_OK;
     CUDA_TRY(cudaMallocHost(out, (size_t)bytes));
     cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, *out) == cudaSuccess && a.devicePointer == *out)
-        HostBlocks::all().add(*out, (size_t)bytes);
+    if (cudaPointerGetAttributes(&a, *out) != cudaSuccess) (void)cudaGetLastError();
+    else if (a.devicePointer == *out) HostBlocks::all().add(*out, (size_t)bytes);
     return FCC_OK;
 }
 fcc_status fcc_host_free(void* ptr) {

@@ -128,3 +128,15 @@ def test_cell_scan_over_its_ranges(nx, ny, n):
     assert a.ncx * a.ncy == b.ncx * b.ncy and s.builds == o.builds
     for f in ("cellid", "perm", "start", "stop", "count"):
         assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
+def test_a_refused_page_lock_does_not_fail_the_next_call():
+    """Page-locked memory that the system does not give (4 PB here) is an error
+    of that request alone: results come in ordinary arrays then, and the calls
+    that follow, kernel launches among them, do not see it."""
+    bodies, box, kw = sim(np.float64)
+    s, lib = fcc.Simulation(bodies, box, **kw), fcc.native_library()
+    p = C.c_void_p()
+    for query in (lambda: s.bodies, s.shape_index, lambda: s.refresh().grad, lambda: s.run(2)):
+        assert lib.fcc_host_alloc(1 << 52, C.byref(p)) == abi.FCC_ERR_NOMEM
+        query()
