@@ -2755,6 +2755,13 @@ __global__ void __launch_bounds__(INIT_BLOCK) k_init(DevPtrs<T> d, int par, int 
                                                     const int* __restrict__ w, const int* __restrict__ ix_in,
                                                     const int* __restrict__ iy_in) {
     extern __shared__ double s_coef[];
+    // the counts are zero between builds, but for a launch that gave up at a
+    // barrier of one: setting the state clears that too
+    if (d.ctot) {
+        const int tid = blockIdx.x * INIT_BLOCK + threadIdx.x, nthr = gridDim.x * INIT_BLOCK;
+        for (int c = tid; c < d.Ctot; c += nthr) d.ccount[c] = 0;
+        for (int r = tid; r * SCAN_RANGE < d.Ctot; r += nthr) d.ctot[r] = 0;
+    }
     const int i0 = blockIdx.x * INIT_BODIES;
     const int nb = min(INIT_BODIES, n - i0);
     const int i = i0 + threadIdx.x;

@@ -89,6 +89,40 @@ extern "C" int unit_roots(const double* x, int n, double* inv, double* root) {
     return (int)dr.back(root);
 }
 
+// k_init of n bodies in a grid of `cells` cells; count[cells] and total[ranges]
+// as the launch finds and leaves them
+extern "C" int unit_init_counts(int n, int cells, int* count, int* total) {
+    SimDesc<double> h{};
+    h.K = KM;
+    h.n = n;
+    h.ncells = cells;
+    for (int t = 0; t < MT; ++t) h.kmax[t] = KM;
+    const std::vector<double> zero((size_t)n * RECW, 0.0), one(n, 1.0);
+    const std::vector<int> izero(n, 0);
+    Dev<SimDesc<double>> P(&h, 1);
+    Dev<double> rec0(zero.data(), (size_t)n * RECW), rec1(zero.data(), (size_t)n * RECW),
+        coef(zero.data(), (size_t)n * NCM), in(zero.data(), (size_t)n * NCM), x(zero.data(), n), r0(one.data(), n);
+    Dev<int> sim_of(izero.data(), n), w(izero.data(), n), c(count, cells), t(total, (cells + SCAN_RANGE - 1) / SCAN_RANGE);
+    for (cudaError_t e : {P.e, rec0.e, rec1.e, coef.e, in.e, x.e, r0.e, sim_of.e, w.e, c.e, t.e}) TRY(e);
+    DevPtrs<double> d{};
+    d.sims = P.p;
+    d.nsims = 1;
+    d.Ntot = n;
+    d.Ctot = cells;
+    d.sim_of = sim_of.p;
+    d.rec0 = rec0.p;
+    d.rec1 = rec1.p;
+    d.coef = coef.p;
+    d.R0 = r0.p;
+    d.ccount = c.p;
+    d.ctot = t.p;
+    k_init<double><<<(n + INIT_BODIES - 1) / INIT_BODIES, INIT_BLOCK, init_smem_bytes(NCM)>>>(
+        d, 0, 0, n, x.p, x.p, x.p, in.p, NCM, KM, w.p, nullptr, nullptr);
+    TRY(cudaGetLastError());
+    TRY(c.back(count));
+    return (int)t.back(total);
+}
+
 extern "C" int unit_user_gradients(int nth, const double* R, const double* R1, const double* R2, double w, double* GR,
                                    double* GD, double* GDD) {
     SimDesc<double> h{};

@@ -79,3 +79,15 @@ def test_fp64_roots_over_the_exponents(unit):
     assert root[0] == 0 and root[5] == np.inf and np.isnan(root[6])
     # below the smallest normal number: within that number's root of the value
     assert (np.abs(root[1:5] - np.sqrt(x[1:5])) <= np.sqrt(tiny)).all()
+
+
+@pytest.mark.parametrize("n,cells", [(1, 1), (5, 512), (70, 1300), (1000, 513)])
+def test_loading_a_state_clears_the_counts_of_an_abandoned_rebuild(unit, n, cells):
+    """A launch that gave up at a barrier between the count and the scatter of a
+    rebuild leaves bodies counted; added to by the next rebuild they would put
+    bodies beyond the sorted list's end.  Loading a state (which also renews the
+    barriers) starts from zero."""
+    count = np.full(cells, 7, np.int32)
+    total = np.full(-(-cells // 512), 9, np.int32)
+    unit("unit_init_counts", n, cells, count, total)
+    assert not count.any() and not total.any()
