@@ -131,10 +131,12 @@ struct Stage {
     V* p() const { return buf.p; }
 };
 
-// The device's address of page-locked host memory that the device reads and
-// writes in place (every page-locked allocation is mapped under unified
-// addressing), or null for any other pointer (pageable memory, device
-// memory, null).
+// The device's address of an array of n elements in page-locked host memory
+// that the device reads and writes in place (every page-locked allocation is
+// mapped under unified addressing), or null for any other pointer (pageable
+// memory, device memory, null) and for arrays that the kernels, which access
+// whole elements, cannot take: misaligned ones, and ones that leave the
+// page-locked range.
 // Blocks of fcc_host_alloc are known by their ranges: their addresses are the
 // device's too, and looking them up costs 0.1 us where the runtime's query
 // takes 0.5 (a state exchange makes twelve).
@@ -153,26 +155,33 @@ struct HostBlocks {
         std::unique_lock<std::shared_mutex> lk(m);
         at.erase((uintptr_t)p);
     }
-    bool holds(const void* p) {
+    bool holds(const void* p, size_t bytes) {
         std::shared_lock<std::shared_mutex> lk(m);
         auto it = at.upper_bound((uintptr_t)p);
         if (it == at.begin()) return false;
         --it;
-        return (uintptr_t)p < it->first + it->second;
+        return (uintptr_t)p + bytes <= it->first + it->second;
     }
 };
 
-template <class V>
-V* mapped_view(V* p) {
-    if (!p) return nullptr;
-    if (HostBlocks::all().holds(p)) return p;
+inline char* device_address(const void* p) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();  // not a pointer the runtime knows: not mapped
         return nullptr;
     }
-    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
-    return static_cast<V*>(a.devicePointer);
+    return a.type == cudaMemoryTypeHost ? static_cast<char*>(a.devicePointer) : nullptr;
+}
+
+template <class V>
+V* mapped_view(V* p, size_t n) {
+    const uintptr_t at = (uintptr_t)p, last = at + std::max(n, (size_t)1) * sizeof(V) - 1;
+    if (!p || at % alignof(V)) return nullptr;
+    if (HostBlocks::all().holds(p, n * sizeof(V))) return p;
+    char* d = device_address(p);
+    // memory is locked by pages: an array within its first one is locked with it
+    if (d && at >> 12 != last >> 12 && device_address((const void*)last) != d + (last - at)) return nullptr;
+    return reinterpret_cast<V*>(d);
 }
 
 // Page-locked output of k_observables, which writes it in place, grown on
@@ -195,7 +204,7 @@ struct ObsArea {
         host = nullptr;
         cap = 0;
         CUDA_TRY(cudaMallocHost(&host, n * sizeof(double)));
-        dev = mapped_view(host);
+        dev = mapped_view(host, n);
         if (!dev) return fail(FCC_ERR_UNSUPPORTED, "page-locked memory is not mapped");
         cap = n;
         return FCC_OK;
@@ -810,7 +819,7 @@ struct Engine final : EngineBase {
         st_h = &pinned->st;
         up_h = &pinned->up;
         ls_h = &pinned->ls;
-        ls_d = mapped_view(ls_h);
+        ls_d = mapped_view(ls_h, 1);
         if (!ls_d) return fail(FCC_ERR_UNSUPPORTED, "page-locked memory is not mapped");
 
         N = sp.N;
@@ -1026,12 +1035,12 @@ struct Engine final : EngineBase {
         const double *px = nullptr, *py = nullptr, *pth = nullptr, *pc = nullptr;
         const int *pix = nullptr, *piy = nullptr;
         if (n) {
-            px = mapped_view(b->x);
-            py = mapped_view(b->y);
-            pth = mapped_view(b->theta);
-            pc = mapped_view(b->coef);
-            pix = mapped_view(b->imgx);
-            piy = mapped_view(b->imgy);
+            px = mapped_view(b->x, n);
+            py = mapped_view(b->y, n);
+            pth = mapped_view(b->theta, n);
+            pc = mapped_view(b->coef, n * nc);
+            pix = mapped_view(b->imgx, n);
+            piy = mapped_view(b->imgy, n);
             const bool in_place = px && py && pth && pc && (!b->imgx || pix) && (!b->imgy || piy);
             if (!in_place) {
                 double* dx = xch_d.p;
@@ -1279,9 +1288,9 @@ struct Engine final : EngineBase {
             if (o->n != N || o->ncoef != nc) return fail(FCC_ERR_DIMENSION, "state buffers do not match the simulation");
             const size_t n = (size_t)N;
             if (n) {
-                double *vx = mapped_view(o->x), *vy = mapped_view(o->y), *vth = mapped_view(o->theta),
-                       *vc = mapped_view(o->coef);
-                int *vix = mapped_view(o->imgx), *viy = mapped_view(o->imgy);
+                double *vx = mapped_view(o->x, n), *vy = mapped_view(o->y, n), *vth = mapped_view(o->theta, n),
+                       *vc = mapped_view(o->coef, n * nc);
+                int *vix = mapped_view(o->imgx, n), *viy = mapped_view(o->imgy, n);
                 const bool in_place = (!o->x || vx) && (!o->y || vy) && (!o->theta || vth) && (!o->coef || vc) &&
                                       (!o->imgx || vix) && (!o->imgy || viy);
                 const int grid = (int)std::min<int64_t>((N * nc + 255) / 256, (int64_t)nsm * 8);
@@ -1355,12 +1364,12 @@ struct Engine final : EngineBase {
         };
         GradOut<T> v = g;
         bool in_place = true;
-        auto view = [&](double* host, double*& dev) {
-            dev = mapped_view(host);
+        auto view = [&](double* host, size_t count, double*& dev) {
+            dev = mapped_view(host, count);
             in_place = in_place && (!host || dev);
         };
-        for (int b = 0; b < 4; ++b) view(node_out[b], v.node_out[b]), view(body_out[b], v.body_out[b]);
-        for (int b = 0; b < 2; ++b) view(coef_out[b], v.coef_out[b]);
+        for (int b = 0; b < 4; ++b) view(node_out[b], n * nth, v.node_out[b]), view(body_out[b], n, v.body_out[b]);
+        for (int b = 0; b < 2; ++b) view(coef_out[b], n * nc, v.coef_out[b]);
         if (in_place) {
             FCC_TRY(store(v));
             return sync_stream();
@@ -1648,7 +1657,7 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
     CUDA_TRY(cudaMemcpyAsync(w->head.p, w->head_h, sizeof(typename ListWork<T>::Head), cudaMemcpyHostToDevice, st));
     // inputs: page-locked ones are read in place, others through page-locked
     // staging (or, in large numbers, a device area)
-    const double *xd = mapped_view(x), *yd = mapped_view(y), *rd = mapped_view(rmax);
+    const double *xd = mapped_view(x, N), *yd = mapped_view(y, N), *rd = mapped_view(rmax, N);
     if (!(xd && yd && rd)) {
         if (N <= ListWork<T>::STAGED) {
             if (w->in_cap < 3 * N) {
@@ -1661,7 +1670,7 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
             std::memcpy(w->in_h, x, N * sizeof(double));
             std::memcpy(w->in_h + N, y, N * sizeof(double));
             std::memcpy(w->in_h + 2 * N, rmax, N * sizeof(double));
-            xd = mapped_view(w->in_h);
+            xd = mapped_view(w->in_h, 3 * N);
         } else {
             if (w->in.n < 3 * N) FCC_TRY(w->in.alloc(3 * N, st));
             CUDA_TRY(cudaMemcpyAsync(w->in.p, x, N * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -1713,7 +1722,7 @@ fcc_status build_neighbors_t(int64_t n, const double* x, const double* y, const 
     bool in_place = true;
     size_t total = 0;
     for (int k = 0; k < 6; ++k) {
-        dev[k] = mapped_view(host[k]);
+        dev[k] = mapped_view(host[k], len[k]);
         in_place = in_place && dev[k];
         total += len[k];
     }

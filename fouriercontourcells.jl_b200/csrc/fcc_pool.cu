@@ -1020,8 +1020,9 @@ struct Pool final : PoolBase {
             if (o->n != N || o->ncoef != P.nc) return fail(FCC_ERR_DIMENSION, "state buffers do not match the simulation");
             Arena<T>& a = *A;
             const size_t n = (size_t)N;
-            double *vx = mapped_view(o->x), *vy = mapped_view(o->y), *vth = mapped_view(o->theta), *vc = mapped_view(o->coef);
-            int *vix = mapped_view(o->imgx), *viy = mapped_view(o->imgy);
+            double *vx = mapped_view(o->x, n), *vy = mapped_view(o->y, n), *vth = mapped_view(o->theta, n),
+                   *vc = mapped_view(o->coef, n * P.nc);
+            int *vix = mapped_view(o->imgx, n), *viy = mapped_view(o->imgy, n);
             const bool in_place = (!o->x || vx) && (!o->y || vy) && (!o->theta || vth) && (!o->coef || vc) &&
                                   (!o->imgx || vix) && (!o->imgy || viy);
             if (n > 0 && in_place) {  // page-locked arrays: written by the kernel, one launch and no copy

@@ -140,3 +140,37 @@ def test_a_refused_page_lock_does_not_fail_the_next_call():
     for query in (lambda: s.bodies, s.shape_index, lambda: s.refresh().grad, lambda: s.run(2)):
         assert lib.fcc_host_alloc(1 << 52, C.byref(p)) == abi.FCC_ERR_NOMEM
         query()
+
+
+def odd(a):
+    """A page-locked array like `a`, half an element off its alignment."""
+    block = simulation._ResultBlocks().take(fcc.native_library(), a.nbytes + 64)
+    v = np.ndarray(a.shape, a.dtype, block, a.itemsize // 2)
+    v[...] = a
+    return v
+
+
+def test_misaligned_page_locked_arrays():
+    """Page-locked arrays off their alignment, which the device cannot access,
+    are copied like ordinary ones: states, gradients and lists equal those
+    through aligned arrays."""
+    bodies, box, kw = sim(np.float64, n=(32, 32))
+    s = fcc.Simulation(bodies, box, **kw).refresh()
+    s.run(3)
+    want, grad = s.bodies, s.refresh().grad
+    GR = odd(np.zeros((s.N, s.nθ)))
+    g = abi.FccGradientsHost(abi.dptr(GR), *[None] * 9)
+    s._call("get_gradients", s._h, C.byref(g))
+    assert np.array_equal(GR.T, grad.GR)
+    b = want.copy()
+    for f in ("x", "y", "θ", "imgx", "imgy"):
+        setattr(b, f, odd(getattr(want, f)))
+    b.coef = odd(np.ascontiguousarray(want.coef.T)).T
+    s.set_state(b)
+    for f in ("x", "y", "θ", "imgx", "imgy", "coef"):
+        getattr(b, f)[...] = 0
+    s.get_state(out=b)
+    for f in ("x", "y", "θ", "imgx", "imgy", "coef"):
+        assert np.array_equal(getattr(b, f), getattr(want, f)), f
+    (x, y, rmax, *rest), kwl = neighbors(3, 4000, np.float64)
+    same(fcc.build_neighbors(odd(x), odd(y), odd(rmax), *rest, **kwl), oracle.build_neighbors(x, y, rmax, *rest, **kwl))
