@@ -19,7 +19,7 @@ import math
 import os
 import threading
 import weakref
-from collections import namedtuple
+from collections import deque, namedtuple
 
 import numpy as np
 
@@ -74,7 +74,10 @@ class _ResultBlocks:
     LIMIT = 256 << 20
 
     def __init__(self):
-        self._lock = threading.RLock()  # a collection may give a block back inside take
+        self._lock = threading.RLock()
+        # blocks whose last array was collected, until the next request sorts
+        # them in: a collection may come at any step of a request
+        self._back = deque()
         self._idle = {}
         self._total = 0
 
@@ -87,6 +90,9 @@ class _ResultBlocks:
         """A uint8 array of at least nbytes, or None."""
         size = self.size_of(max(1, nbytes))
         with self._lock:
+            while self._back:
+                ptr, n = self._back.popleft()
+                self._idle.setdefault(n, []).append(ptr)
             idle = self._idle.get(size)
             if idle:
                 ptr = idle.pop()
@@ -105,8 +111,7 @@ class _ResultBlocks:
         return block
 
     def _give(self, ptr, size):
-        with self._lock:
-            self._idle.setdefault(size, []).append(ptr)
+        self._back.append((ptr, size))
 
 
 _BLOCKS = _ResultBlocks()
