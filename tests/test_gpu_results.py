@@ -174,3 +174,19 @@ def test_misaligned_page_locked_arrays():
         assert np.array_equal(getattr(b, f), getattr(want, f)), f
     (x, y, rmax, *rest), kwl = neighbors(3, 4000, np.float64)
     same(fcc.build_neighbors(odd(x), odd(y), odd(rmax), *rest, **kwl), oracle.build_neighbors(x, y, rmax, *rest, **kwl))
+
+
+def test_gradients_into_ordinary_memory_keep_their_device_area():
+    """Queries of gradients into a caller's own arrays allocate device memory
+    once: what the first one took is still held after it, and later ones take
+    no more."""
+    import torch
+    bodies, box, kw = sim(np.float64, n=(128, 128), nθ=40)
+    s = fcc.Simulation(bodies, box, **kw).refresh()
+    P = np.zeros((s.N, s.nθ))
+    g = abi.FccGradientsHost(None, None, None, abi.dptr(P), *[None] * 6)
+    free = [torch.cuda.mem_get_info()[0]]
+    for _ in range(3):
+        s._call("get_gradients", s._h, C.byref(g))
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] >= P.nbytes - (2 << 20) and free[1] == free[2] == free[3]
