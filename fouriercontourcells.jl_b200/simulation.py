@@ -14,6 +14,7 @@ and fails loudly when that library is missing: there is no CPU fallback.
 
 from __future__ import annotations
 
+import bisect
 import ctypes as C
 import math
 import os
@@ -61,70 +62,186 @@ def native_library():
     return _LIB
 
 
+class _Slab:
+    """One page-locked allocation: its address, size and holes, sorted by
+    offset as [offset, length]."""
+
+    def __init__(self, at, size):
+        self.at, self.size, self.holes = at, size, [[0, size]]
+
+    def carve(self, size):
+        for k, hole in enumerate(self.holes):
+            if hole[1] >= size:
+                at = self.at + hole[0]
+                hole[0] += size
+                hole[1] -= size
+                if not hole[1]:
+                    del self.holes[k]
+                return at
+        return None
+
+    def restore(self, ptr, size):
+        off = ptr - self.at
+        k = bisect.bisect(self.holes, [off])
+        self.holes.insert(k, [off, size])
+        if k + 1 < len(self.holes) and off + size == self.holes[k + 1][0]:
+            self.holes[k][1] += self.holes.pop(k + 1)[1]
+        if k and sum(self.holes[k - 1]) == off:
+            self.holes[k - 1][1] += self.holes.pop(k)[1]
+
+
 class _ResultBlocks:
     """Page-locked memory of the arrays that queries return (states, gradient
     buffers, neighbour lists), which the device then writes in place: the
     kernel that widens and repacks a result writes it across PCIe once, with
     no staging copy and no host pass.  A block goes back when the last array
-    over it is collected and is handed out again for the next result of its
-    size.  At most ``LIMIT`` bytes are page-locked at a time, blocks in use
-    included (a program that keeps every snapshot gets ordinary arrays beyond
-    that: ``take`` returns None)."""
+    over it is collected and is handed out again.
+
+    Page-locking costs some ms, more than the copy of one result, so a query
+    does not pay for it before it is worth it: results are ordinary arrays
+    until those that came back (collected, so that their memory could have
+    served again) would have saved twice its price (``saving``, ``price``).
+    A program that keeps every result never pays; one that drops them pays
+    once, after some six results of 7 MB.  Measured for the gradient buffers of
+    4096 bodies (7 MB): a first result 3.2 to 5.8 ms with the lock in the query,
+    1.1 in ordinary arrays, 0.18 in a block that came back; for the state of
+    16384 bodies (3.3 MB) 5.3, 1.6 and 0.09.  Blocks are cut from slabs; results
+    of up to ``SLAB`` bytes share them, larger ones have slabs, and a reckoning,
+    of their size.  At most ``LIMIT`` bytes are page-locked at a time, those in
+    use included."""
 
     LIMIT = 256 << 20
+    SLAB = 4 << 20
 
     def __init__(self):
         self._lock = threading.RLock()
-        # blocks whose last array was collected, until the next request sorts
-        # them in: a collection may come at any step of a request
+        # what was collected since the last request: (address, size) of a
+        # block, (None, size) of an ordinary result; a collection may come at
+        # any step of a request
         self._back = deque()
-        self._idle = {}
+        self._idle = {}    # size: addresses of blocks of that size, cut already
+        self._slabs = []
         self._total = 0
+        self._credit = {}  # slab size: us that results which came back would have saved
+        self._busy = False
 
     @staticmethod
     def size_of(nbytes: int) -> int:
         step = 1 << max(12, nbytes.bit_length() - 4)  # at most one eighth wasted
         return -(-nbytes // step) * step
 
-    def take(self, lib, nbytes: int):
-        """A uint8 array of at least nbytes, or None."""
+    @staticmethod
+    def saving(size: int) -> float:
+        """us that a result in place saves: calls and the copy (measured 80 us at
+        11 kB, 0.9 ms at 7 MB, 10 ms at 52 MB)."""
+        return 80 + 0.2e-3 * size
+
+    @staticmethod
+    def price(size: int) -> float:
+        """us of page-locking a slab (measured 1.2 to 1.7 ms at 1 MB, 5 at 7 MB, 24
+        at 64 MB)."""
+        return 1000 + 0.4e-3 * size
+
+    def _sort_in(self):
+        while self._back:
+            ptr, size = self._back.popleft()
+            if ptr is None:
+                slab = max(size, self.SLAB)
+                self._credit[slab] = self._credit.get(slab, 0.0) + self.saving(size)
+            else:
+                self._idle.setdefault(size, []).append(ptr)
+
+    def _find(self, size):
+        """The address of a free block, or None."""
+        idle = self._idle.get(size)
+        if idle:
+            return idle.pop()
+        for other, ptrs in list(self._idle.items()):  # blocks of other sizes become holes
+            while ptrs:
+                ptr = ptrs.pop()
+                next(s for s in self._slabs if s.at <= ptr < s.at + s.size).restore(ptr, other)
+        for slab in self._slabs:
+            ptr = slab.carve(size)
+            if ptr is not None:
+                return ptr
+        return None
+
+    def _grow(self, lib, size) -> bool:
+        """Page-lock a slab that holds a block of `size`, in place of idle ones
+        where ``LIMIT`` needs that."""
+        free = [s for s in self._slabs if s.holes == [[0, s.size]]]
+        if self._total + size - sum(s.size for s in free) > self.LIMIT:
+            return False
+        while self._total + size > self.LIMIT:
+            slab = free.pop()
+            self._slabs.remove(slab)
+            self._total -= slab.size
+            lib.fcc_host_free(slab.at)
+        p, room = C.c_void_p(), max(size, min(self.SLAB, self.LIMIT - self._total))
+        if lib.fcc_host_alloc(room, C.byref(p)) != abi.FCC_OK:
+            return False
+        self._slabs.append(_Slab(p.value, room))
+        self._total += room
+        return True
+
+    def take(self, lib, nbytes: int, worth: bool = False):
+        """A uint8 array of at least nbytes in page-locked memory, or None.
+        `worth`: page-lock more only where that is worth it."""
         size = self.size_of(max(1, nbytes))
         with self._lock:
-            while self._back:
-                ptr, n = self._back.popleft()
-                self._idle.setdefault(n, []).append(ptr)
-            idle = self._idle.get(size)
-            if idle:
-                ptr = idle.pop()
-            else:
-                while self._total + size > self.LIMIT and any(self._idle.values()):
-                    other = next(k for k, v in self._idle.items() if v)
-                    lib.fcc_host_free(self._idle[other].pop())
-                    self._total -= other
-                p = C.c_void_p()
-                if self._total + size > self.LIMIT or lib.fcc_host_alloc(size, C.byref(p)) != abi.FCC_OK:
-                    return None
-                ptr = p.value
-                self._total += size
+            if self._busy:  # the query of a finaliser that a collection runs inside this one
+                return None
+            self._busy = True
+            try:
+                ptr = self._address(lib, size, worth)
+            finally:
+                self._busy = False
+        if ptr is None:
+            return None
         block = np.frombuffer((C.c_uint8 * size).from_address(ptr), dtype=np.uint8)
-        weakref.finalize(block, self._give, ptr, size).atexit = False
+        weakref.finalize(block, self._back.append, (ptr, size)).atexit = False
         return block
 
-    def _give(self, ptr, size):
-        self._back.append((ptr, size))
+    def _address(self, lib, size, worth):
+        self._sort_in()
+        ptr = self._find(size)
+        if ptr is None:
+            slab = max(size, self.SLAB)
+            if worth and self._credit.get(slab, 0.0) < 2 * self.price(slab):
+                return None
+            self._credit.pop(slab, None)
+            if self._grow(lib, size):
+                ptr = self._find(size)
+        return ptr
+
+    def ordinary(self, array, nbytes: int):
+        """Take note of an ordinary result of nbytes, `array` a part of it."""
+        weakref.finalize(array, self._back.append, (None, self.size_of(max(1, nbytes)))).atexit = False
 
 
 _BLOCKS = _ResultBlocks()
 
 
+def _result_block(lib, nbytes):
+    """Page-locked memory for a result, and what to call with an ordinary array
+    where there is none."""
+    if not hasattr(lib, "fcc_host_alloc"):
+        return None, lambda array: None
+    return _BLOCKS.take(lib, nbytes, worth=True), lambda array: _BLOCKS.ordinary(array, nbytes)
+
+
 def result_arrays(lib, *shapes):
-    """Arrays, one per (shape, dtype), for the library to fill: over one
-    page-locked block where there is room for it (their contents are then
-    whatever the block held), else zeros."""
+    """Arrays, one per (shape, dtype), for the library to fill, over one
+    page-locked block where there is one to be had."""
     sizes = [math.prod(shape) * dt().itemsize for shape, dt in shapes]
-    block = _BLOCKS.take(lib, sum(-(-n // 64) * 64 for n in sizes)) if hasattr(lib, "fcc_host_alloc") else None
+    total = sum(-(-n // 64) * 64 for n in sizes)
+    block, ordinary = _result_block(lib, total)
     if block is None:
-        return [np.zeros(shape, dt) for shape, dt in shapes]
+        # the CUDA library writes every element; another may leave unused ones
+        new = np.empty if hasattr(lib, "fcc_host_alloc") else np.zeros
+        out = [new(shape, dt) for shape, dt in shapes]
+        ordinary(out[0])
+        return out
     out, off = [], 0
     for (shape, dt), n in zip(shapes, sizes):
         out.append(block[off:off + n].view(dt).reshape(shape))
@@ -138,10 +255,17 @@ def result_bodies(lib, n: int, ncoef: int):
     d, k = -(-8 * n // 64) * 64, -(-4 * n // 64) * 64  # bytes of a vector of doubles, of ints
     # x, y, θ, R0, the ints, then the coefficients
     ends = [0, d, 2 * d, 3 * d, 4 * d, 4 * d + k, 4 * d + 2 * k, 4 * d + 3 * k, 4 * d + 4 * k]
-    block = _BLOCKS.take(lib, ends[8] + 8 * n * ncoef) if hasattr(lib, "fcc_host_alloc") else None
-    if block is None:
-        block = np.zeros(ends[8] + 8 * n * ncoef, np.uint8)
+    total = ends[8] + 8 * n * ncoef
     f, i, new = np.float64, np.int32, np.ndarray
+    block, ordinary = _result_block(lib, total)
+    if block is None:
+        x, y, θ, R0 = (np.empty(n, f) for _ in range(4))
+        imgx, imgy, typ, parent = (np.empty(n, i) for _ in range(4))
+        rows = np.empty((n, ncoef), f)
+        ordinary(rows)
+        host = abi.bodies_host_at(n, ncoef, *(v.__array_interface__["data"][0] for v in (
+            x, y, θ, imgx, imgy, rows, R0, typ, parent)))
+        return Bodies(x, y, θ, imgx, imgy, rows.T, R0, typ, parent), host
     x, y, θ, R0 = (new(n, f, block, o) for o in ends[:4])
     imgx, imgy, typ, parent = (new(n, i, block, o) for o in ends[4:8])
     coef = new((n, ncoef), f, block, ends[8]).T

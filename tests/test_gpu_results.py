@@ -176,6 +176,32 @@ def test_misaligned_page_locked_arrays():
     same(fcc.build_neighbors(odd(x), odd(y), odd(rmax), *rest, **kwl), oracle.build_neighbors(x, y, rmax, *rest, **kwl))
 
 
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+def test_results_change_to_page_locked_memory(T, monkeypatch):
+    """The same query again and again, its results dropped: ordinary arrays
+    first, page-locked ones once enough came back, equal values throughout, for
+    gradients, states, pool states and neighbour lists."""
+    bodies, box, kw = sim(T, n=(32, 32))
+    s = fcc.Simulation(bodies, box, **kw).refresh()
+    s.run(3)
+    s.refresh()
+    nθ = kw.pop("nθ")
+    pool = fcc.Pool(nθ=nθ, T=kw.pop("T"), max_bodies=2048, max_cells=2048, max_sims=2)
+    slot = pool.add(bodies, box, horizon=1 << 20, **kw)
+    pool.run(3)
+    args, kwl = neighbors(5, 4000, T)
+    for query in (lambda: list(s.grad), lambda: [getattr(s.bodies, f) for f in ("x", "y", "θ", "coef", "imgx", "R0", "type")],
+                  lambda: [getattr(pool.bodies(slot), f) for f in ("x", "y", "θ", "coef", "imgy", "R0", "parent")],
+                  lambda: list(fcc.build_neighbors(*args, **kwl))):
+        monkeypatch.setattr(simulation, "_BLOCKS", simulation._ResultBlocks())
+        first, places = query(), []
+        for _ in range(200):
+            got = query()
+            assert all(np.array_equal(a, b) for a, b in zip(first, got))
+            places.append(any(v.at <= got[0].ctypes.data < v.at + v.size for v in simulation._BLOCKS._slabs))
+        assert not places[0] and places[-1] and places == sorted(places)
+
+
 def test_gradients_into_ordinary_memory_keep_their_device_area():
     """Queries of gradients into a caller's own arrays allocate device memory
     once: what the first one took is still held after it, and later ones take
