@@ -253,6 +253,10 @@ const Variant VARIANTS[] = {
     {8, 5, 224, 2, step_fn<float, 8, 5, 224, 2>, step_fn<double, 8, 5, 224, 2>, stage_bytes_per_warp<float, 8, 5>(),
      stage_bytes_per_warp<double, 8, 5>(), 0},
     {8, 5, 256, 1, step_fn<float, 8, 5, 256, 1>, nullptr, stage_bytes_per_warp<float, 8, 5>(), 0, 0},
+    // contours of 41 to 64 nodes in one chunk: the bits of family 0's two chunks
+    // (a lane's nodes and every sum in the same order; tested alone and against
+    // pools), but of a family of its own: the tuner's default candidates are the
+    // shapes of 5 nodes a lane
     {8, 8, 256, 1, nullptr, step_fn_one<double, 8, 8, 256, 1>, 0, stage_bytes_per_warp<double, 8, 8>(), 4},
 };
 constexpr int NVARIANTS = sizeof(VARIANTS) / sizeof(VARIANTS[0]);

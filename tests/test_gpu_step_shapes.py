@@ -218,3 +218,25 @@ def test_a_tuned_shape_does_not_bind_other_contours():
     a, b = alone.bodies, pool.bodies(slot)
     for f in ("x", "y", "θ", "coef"):
         assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
+@pytest.mark.parametrize("nθ", [48, 64])
+def test_finer_contours_in_a_pool_of_two_rounds_equal_lone_runs(nθ):
+    """FP64 contours of 41 to 64 nodes: members of a pool of more bodies than one
+    round holds (two chunks, two blocks per SM) against the same simulations
+    alone (one chunk of 8 nodes a lane), over many rebuilds: the same bits."""
+    pool = fcc.Pool(T=np.float64, nθ=nθ, max_bodies=8192, max_cells=8192, max_sims=8)
+    lone, slots = [], []
+    for k in range(5):
+        bodies, box = deformed(32, 32 + 2 * k, 10, 40 + k)
+        kw = {**KW, "types": (fcc.BodyType(v0=0.3, Dr=0.2, Dt=0.02, μab=0.1),), "seed": 3 + k}
+        slots.append(pool.add(bodies, box, horizon=1 << 20, **kw))
+        lone.append(fcc.Simulation(bodies, box, T=np.float64, nθ=nθ, **kw))
+    assert sum(s.N for s in lone) > 4736 and pool.variant()["slots"] == 5
+    pool.run(300)
+    for s, slot in zip(lone, slots):
+        s.run(300)
+        assert s.builds > 10 and pool.builds(slot) == s.builds
+        a, b = s.bodies, pool.bodies(slot)
+        for f in ("x", "y", "θ", "coef"):
+            assert np.array_equal(getattr(a, f), getattr(b, f)), f
