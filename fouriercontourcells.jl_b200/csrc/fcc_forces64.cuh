@@ -2,9 +2,9 @@
 //
 // Same work per body as the FP32 forces_warp (fcc_kernels.cuh), arranged for
 // the FP64 units.  8 lanes per body, 4 bodies per warp; lane l of a body owns
-// the contour nodes l + 8 s, s < 5, of a chunk and the modes m = l (and lane
-// 0 m = 8 too).  The contractions over modes and nodes run on the FP64 tensor
-// cores (mma.sync m8n8k4, IEEE double products and sums):
+// the contour nodes l + 8 s, s < S (5, or 8 in variant 7), of a chunk and the
+// modes m = l (and lane 0 m = 8 too).  The contractions over modes and nodes run
+// on the FP64 tensor cores (mma.sync m8n8k4, IEEE double products and sums):
 //   synthesis  [R_b ; R'_b] (8 rows) = [c_b ; c'_b] (8 x 20) . M^T (20 x 8 S)
 //   pullback   [g_b ; h_b]  (8 rows) = [GR_b ; GD_b] (8 x 8 S) . M (8 S x 20)
 // with rows 2b + h (b the body, h = bit 2 of the lane: value or derivative),

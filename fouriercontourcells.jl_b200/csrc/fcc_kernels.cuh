@@ -691,8 +691,10 @@ constexpr int MMA_TABLE_FLOATS = (MMA_SYN_TILES + MMA_PB_TILES) * 2 * 32 * 4;
 // FP64 (fcc_forces64.cuh): columns of the contraction matrix, its rows after
 // the last node, neighbour records staged per body and doubles between staged
 // records (208 bytes: the 16-byte reads of a warp's lanes at different
-// neighbours fall into different banks).  With NBMAX64 = 10 two blocks of 224
-// threads fit an SM's shared memory (14 warps); 12 would not.
+// neighbours fall into different banks).  8 records: one neighbour id a lane,
+// 8 slots x 8 neighbours in one 64-bit hit mask, and the shared memory of two
+// blocks of 224 threads (12 records would not fit); a body with more listed
+// neighbours stages them in batches of 8.
 constexpr int M64_COLS = 20, M64_PAD = 80, NBMAX64 = 8, SREC64 = RECW + 2;
 // own body-frame coefficients, sin and cos of theta, 1/(2 a0)
 constexpr int SCF64 = NCM + 3;
@@ -1524,6 +1526,7 @@ __device__ __forceinline__ void contact_lat(const T* snb, int n, int q0, int q1,
 // USER: the simulation has compiled user terms (include/fcc_user_terms.h):
 // R'' is synthesised, user integrals, node gradients (GDD included),
 // pressures and bond gradients are added, and the pullback includes R''.
+// Only T = float is instantiated (forces_group sends double to forces_warp64).
 template <class T, int L, int S, bool ONE, int MODE, bool USER = false, bool LAT = false>
 __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stage, int par, const SimDesc<T>* sim0,
                                             const T* tab, int& cached, int* rbp, const BarrierLocal* lone, bool drawn, Resident<T, L>* res = nullptr) {
@@ -2090,7 +2093,9 @@ __device__ __forceinline__ void forces_warp(const DevPtrs<T>& d, int wg, T* stag
         lane_mode_grads<T, L>(gl, l, gA, gB);
     }
 
-    // ---- bond forces on the centre (every lane of the body, no shuffles)
+    // ---- bond forces on the centre (every lane of the body, no shuffles): as
+    // bond_forces, kept in place for the FP32 kernels' bits and registers; so are
+    // the user body terms above (UserBody): a change to a term is made in both
     if (act && (P.nbd > 0 || (USER && P.nubd > 0))) {
         const int bc = __ldg(d.bd_count + g);
         T bx = T(0), by = T(0);
@@ -2702,9 +2707,10 @@ __global__ void k_prepare_rebuild(DevPtrs<T> d, int force) {
 
 // The rebuild of update_neighbors! for a simulation of its own, as decided by
 // k_prepare_rebuild: the step kernel's phases and barriers in one cooperative
-// launch instead of one each and a copy of the status (FP64, 4096 bodies: state
-// in, rebuild, forces and all gradient buffers out 296 us, with this 279).  The last block to end leaves the flags for the next step (which
-// rebuilds again only with skin = 0) and the status for the host.
+// launch instead of one each and a copy of the status (FP64, 4096 bodies, state
+// in, rebuild, forces and all gradient buffers out: 296 us a pass before, 279
+// with this kernel).  The last block to end leaves the flags for the next step
+// (which rebuilds again only with skin = 0) and the status for the host.
 constexpr int REBUILD_BLOCK = 256;
 template <class T>
 __global__ void __launch_bounds__(REBUILD_BLOCK) k_rebuild(DevPtrs<T> d, int par, LaunchStatus* status,
