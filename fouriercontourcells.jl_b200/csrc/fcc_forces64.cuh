@@ -437,15 +437,14 @@ __device__ __forceinline__ void forces_warp64(const DevPtrs<double>& d, int wg, 
     for (int ch = 0; ch < nch; ++ch) {
         synth(ch);
 #pragma unroll
-        for (int sl = 0; sl < S; ++sl) {  // nodes beyond the contour: no branch, their value is dropped
-            const bool v = vmask & (1u << sl);
-            // the smallest normal number is lost in any sum but at R = R' = 0 (a
-            // shape at its bound may touch the centre), where the root of 0 is 0
-            // to 1e-154 instead of 0 times infinity; it costs no instruction (a
-            // comparison a node: 884 against 904 us a pass of 1024 bodies)
+        for (int sl = 0; sl < S; ++sl) {
+            // the smallest normal number is lost in any sum but at R = R' = 0: a node
+            // beyond the contour, or one where a shape at its bound touches the
+            // centre.  There it makes the root of 0 0 to 1e-154, where x times its
+            // reciprocal root is 0 times infinity, at no cost (1024 bodies 877 -> 875
+            // us a pass; with a mask a node 882 -> 889, with a comparison 885 -> 904)
             const T x2 = fma(R[sl], R[sl], fma(R1[sl], R1[sl], T(2.2250738585072014e-308)));
-            const T q = x2 * rsqrt_normal(v ? x2 : T(1));
-            Qp += v ? q : T(0);
+            Qp = add_rn(Qp, mul_rn(x2, rsqrt_normal(x2)));  // not fused: every launch shape the same bits
         }
     }
     const T Q = group_sum<L>(Qp) * dphi;
