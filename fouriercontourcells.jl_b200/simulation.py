@@ -193,7 +193,10 @@ class _ResultBlocks:
                 return None
             self._busy = True
             try:
-                ptr = self._address(lib, size, worth)
+                if self._back:
+                    self._sort_in()
+                idle = self._idle.get(size)
+                ptr = idle.pop() if idle else self._address(lib, size, worth)
             finally:
                 self._busy = False
         if ptr is None:
@@ -203,7 +206,7 @@ class _ResultBlocks:
         return block
 
     def _address(self, lib, size, worth):
-        self._sort_in()
+        """The address of a block that is not one of the idle ones of its size."""
         ptr = self._find(size)
         if ptr is None:
             slab = max(size, self.SLAB)
@@ -222,25 +225,17 @@ class _ResultBlocks:
 _BLOCKS = _ResultBlocks()
 
 
-def _result_block(lib, nbytes):
-    """Page-locked memory for a result, and what to call with an ordinary array
-    where there is none."""
-    if not hasattr(lib, "fcc_host_alloc"):
-        return None, lambda array: None
-    return _BLOCKS.take(lib, nbytes, worth=True), lambda array: _BLOCKS.ordinary(array, nbytes)
-
-
 def result_arrays(lib, *shapes):
     """Arrays, one per (shape, dtype), for the library to fill, over one
     page-locked block where there is one to be had."""
     sizes = [math.prod(shape) * dt().itemsize for shape, dt in shapes]
     total = sum(-(-n // 64) * 64 for n in sizes)
-    block, ordinary = _result_block(lib, total)
+    if not hasattr(lib, "fcc_host_alloc"):  # not the CUDA library, which writes every element
+        return [np.zeros(shape, dt) for shape, dt in shapes]
+    block = _BLOCKS.take(lib, total, worth=True)
     if block is None:
-        # the CUDA library writes every element; another may leave unused ones
-        new = np.empty if hasattr(lib, "fcc_host_alloc") else np.zeros
-        out = [new(shape, dt) for shape, dt in shapes]
-        ordinary(out[0])
+        out = [np.empty(shape, dt) for shape, dt in shapes]
+        _BLOCKS.ordinary(out[0], total)
         return out
     out, off = [], 0
     for (shape, dt), n in zip(shapes, sizes):
@@ -257,12 +252,14 @@ def result_bodies(lib, n: int, ncoef: int):
     ends = [0, d, 2 * d, 3 * d, 4 * d, 4 * d + k, 4 * d + 2 * k, 4 * d + 3 * k, 4 * d + 4 * k]
     total = ends[8] + 8 * n * ncoef
     f, i, new = np.float64, np.int32, np.ndarray
-    block, ordinary = _result_block(lib, total)
+    native = hasattr(lib, "fcc_host_alloc")
+    block = _BLOCKS.take(lib, total, worth=True) if native else None
     if block is None:
         x, y, θ, R0 = (np.empty(n, f) for _ in range(4))
         imgx, imgy, typ, parent = (np.empty(n, i) for _ in range(4))
         rows = np.empty((n, ncoef), f)
-        ordinary(rows)
+        if native:
+            _BLOCKS.ordinary(rows, total)
         host = abi.bodies_host_at(n, ncoef, *(v.__array_interface__["data"][0] for v in (
             x, y, θ, imgx, imgy, rows, R0, typ, parent)))
         return Bodies(x, y, θ, imgx, imgy, rows.T, R0, typ, parent), host
